@@ -141,7 +141,8 @@ __device__ __forceinline__ int ghost_rule(const StepArgs &a, const int *g, int *
         int c = cur[d];
         if (d < L::D && a.periodic[d]) {
           const int n = a.dhi[d] - a.dlo[d] + 1;
-          c = a.dlo[d] + (((c - a.dlo[d]) % n) + n) % n;
+          while (c < a.dlo[d]) c += n;  // a ghost lies a cell or two outside
+          while (c > a.dhi[d]) c -= n;
         }
         src[d] = c;
       }
@@ -163,7 +164,9 @@ __device__ __forceinline__ int ghost_rule(const StepArgs &a, const int *g, int *
       else if (cur[d] > a.dhi[d] && a.bchi[d] == ILBM_BC_FOEXTRAP) dsel = d;
     }
     if (dsel < 0) break;
-    cur[dsel] = (cur[dsel] < a.dlo[dsel]) ? a.dlo[dsel] : a.dhi[dsel];
+#pragma unroll
+    for (int d = 0; d < L::D; ++d)  // (constant subscripts: cur stays in registers)
+      if (d == dsel) cur[d] = (cur[d] < a.dlo[d]) ? a.dlo[d] : a.dhi[d];
   }
   src[0] = min(max(g[0], a.dlo[0]), a.dhi[0]);
   src[1] = min(max(g[1], a.dlo[1]), a.dhi[1]);
@@ -178,41 +181,46 @@ __device__ __forceinline__ int ghost_rule(const StepArgs &a, const int *g, int *
 // post-collision value.  Ghosts that are periodic images (self-fill) and
 // halfway bounce-back ghosts are left to the owning cells' push.  A ghost cell
 // is owned by the slab of its lowest dimension outside the box (periodic
-// dimensions excluded in self-fill mode, whose slabs do nothing).
+// dimensions excluded in self-fill mode, whose slabs do not exist), so the
+// shell is one sequence of cells: slab d holds the cells outside the box in
+// dimension d, inside it in the active dimensions below d, and on the grown
+// range of the others (StepArgs::goff, filled by ghost_offsets).
 // The work runs in the leading blocks of the k_step launch (it writes only
 // slots that no cell's push writes, and reads only f^n), so its strided
-// accesses overlap the main stream instead of preceding it.
+// accesses overlap the main stream instead of preceding it.  It is bound by
+// latency: one thread's chain is one ghost's index, its loads in flight
+// together, and its stores.  A thread that walked the 2 D slabs one after
+// another, each with 64-bit index divisions and a load per direction before
+// its store, was the tail of every small launch: a 50 x 50 x 45 FP64 box with
+// covered ghosts took 61 us against 5 us of traffic, and twelve of them 774 us
+// against 320 us with one ghost per thread; the three-level 1024 x 512
+// cylinder 213 -> 182 us per coarse step.  Loading only the entering
+// directions of a copied ghost matters too: all 19 made the two-level sphere
+// 1.3% slower than before instead of 1.3% faster.
+template <class L>
+__device__ __forceinline__ bool ghost_active(const StepArgs &a, int d) {
+  return !(a.self_fill && a.periodic[d]);
+}
+
 template <class L, int S>
-__device__ __noinline__ void ghost_push(const StepArgs &a, int64_t gid, int64_t gstride) {
+__device__ __noinline__ void ghost_push(const StepArgs &a, uint32_t gid, uint32_t gstride) {
   using T = typename Store<S>::T;
   using R = typename Store<S>::R;
-  for (int slab = 0; slab < 2 * L::D; ++slab) {
-  const int d = slab >> 1, side = slab & 1;
-  if (a.self_fill && a.periodic[d]) continue;
-  int ext[3], base[3];
-#pragma unroll
-  for (int e = 0; e < 3; ++e) {
-    if (e >= L::D) { ext[e] = 1; base[e] = 0; continue; }
-    ext[e] = a.hi[e] - a.lo[e] + 3;
-    base[e] = a.lo[e] - 1;
-  }
-  ext[d] = 1;
-  base[d] = side ? a.hi[d] + 1 : a.lo[d] - 1;
-  const int64_t n = (int64_t)ext[0] * ext[1] * ext[2];
   T *fo = static_cast<T *>(a.f_out);
-  for (int64_t t = gid; t < n; t += gstride) {
-    int g[3];
-    g[0] = base[0] + (int)(t % ext[0]);
-    g[1] = base[1] + (int)((t / ext[0]) % ext[1]);
-    g[2] = base[2] + (int)(t / ((int64_t)ext[0] * ext[1]));
-    // owner: lowest dimension outside the box whose slab is active (in
-    // self-fill mode periodic slabs are skipped)
-    int owner = -1;
+  const uint32_t total = a.goff[3];
+  for (uint32_t t = gid; t < total; t += gstride) {
+    const int d = (int)(t >= a.goff[1]) + (int)(L::D == 3 && t >= a.goff[2]);
+    uint32_t r = t - (d == 0 ? 0u : (d == 1 ? a.goff[1] : a.goff[2]));
+    int g[3] = {0, 0, 0};
 #pragma unroll
-    for (int e = 0; e < L::D; ++e)
-      if (owner < 0 && (g[e] < a.lo[e] || g[e] > a.hi[e]) && !(a.self_fill && a.periodic[e]))
-        owner = e;
-    if (owner != d) continue;
+    for (int e = 0; e < L::D; ++e) {
+      const bool inner = e < d && ghost_active<L>(a, e);
+      const uint32_t n = (uint32_t)(a.hi[e] - a.lo[e] + 1);
+      const uint32_t ext = (e == d) ? 2u : (inner ? n : n + 2u);
+      const uint32_t c = (e == L::D - 1) ? r : r % ext;
+      r /= ext;
+      g[e] = (e == d) ? (c ? a.hi[e] + 1 : a.lo[e] - 1) : a.lo[e] + (int)c - (inner ? 0 : 1);
+    }
     // classify the ghost against the domain
     bool phys = false, pure_u1 = true;
 #pragma unroll
@@ -245,7 +253,8 @@ __device__ __noinline__ void ghost_push(const StepArgs &a, int64_t gid, int64_t 
       for (int e = 0; e < L::D; ++e)
         if (a.periodic[e]) {
           const int nn = a.dhi[e] - a.dlo[e] + 1;
-          gw[e] = a.dlo[e] + (((gw[e] - a.dlo[e]) % nn) + nn) % nn;
+          while (gw[e] < a.dlo[e]) gw[e] += nn;
+          while (gw[e] > a.dhi[e]) gw[e] -= nn;
         }
       bool covered = false;
       for (int b = 0; b < a.nlb && !covered; ++b)
@@ -254,6 +263,22 @@ __device__ __noinline__ void ghost_push(const StepArgs &a, int64_t gid, int64_t 
       mode = covered ? 2 : 0;  // not covered: coarse-fine ghost, as given
     }
     const int64_t sb = fidx(a, src[0], src[1], L::D == 3 ? src[2] : 0);
+    // the directions that enter the box, and the loads the ghost needs (those
+    // directions; all of them where moments are formed), in flight together
+    bool into[3][3];
+#pragma unroll
+    for (int e = 0; e < 3; ++e)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const int x = ((e == 2) ? gk : g[e]) + c - 1;
+        into[e][c] = x >= a.lo[e] && x <= a.hi[e];
+      }
+    auto enters = [&](int q) {
+      return into[0][L::cx(q) + 1] && into[1][L::cy(q) + 1] && into[2][L::cz(q) + 1];
+    };
+    R fs[L::Q];
+#pragma unroll
+    for (int q = 0; q < L::Q; ++q) fs[q] = (mode != 0 || enters(q)) ? ldf<L, S>(a, sb, q) : R(0);
     // per-ghost state for the NEQ formula / the collision
     double r64 = 0, u64 = 0, v64 = 0, w64 = 0, rt64 = 0, ut64 = 0, vt64 = 0, wt64 = 0;
     float dr32 = 0, u32 = 0, v32 = 0, w32 = 0, drt32 = 0, ut32 = 0, vt32 = 0, wt32 = 0;
@@ -266,7 +291,7 @@ __device__ __noinline__ void ghost_push(const StepArgs &a, int64_t gid, int64_t 
         double rhonp = 0.0, unp = 0.0, vnp = 0.0, wnp = 0.0;
 #pragma unroll
         for (int p = 0; p < L::Q; ++p) {
-          const double fp = ldf<L, S>(a, sb, p);
+          const double fp = fs[p];
           rhonp = X::add(rhonp, fp);
           unp = X::add(unp, X::mul(double(L::cx(p)), fp));
           vnp = X::add(vnp, X::mul(double(L::cy(p)), fp));
@@ -288,7 +313,7 @@ __device__ __noinline__ void ghost_push(const StepArgs &a, int64_t gid, int64_t 
         float rr = 0.f, m1 = 0.f, m2 = 0.f, m3 = 0.f;
 #pragma unroll
         for (int p = 0; p < L::Q; ++p) {
-          const float gp = ldf<L, S>(a, sb, p);
+          const float gp = fs[p];
           rr += gp;
           if (L::cx(p)) m1 += float(L::cx(p)) * gp;
           if (L::cy(p)) m2 += float(L::cy(p)) * gp;
@@ -322,27 +347,20 @@ __device__ __noinline__ void ghost_push(const StepArgs &a, int64_t gid, int64_t 
           w32 = (L::D == 3) ? ldm<float>(a.macro_in, m + 3 * a.ms2) : 0.0f;
         }
       } else if (S == ILBM_STORAGE_F64) {
-        double fg[L::Q];
-#pragma unroll
-        for (int p = 0; p < L::Q; ++p) fg[p] = ldf<L, S>(a, sb, p);
         double px, py, pz;
         load_force<L, double>(a, a.force_prev, g[0], g[1], gk, px, py, pz);
-        moments64<L>(fg, px, py, pz, r64, u64, v64, w64);
+        moments64<L>(reinterpret_cast<const double *>(fs), px, py, pz, r64, u64, v64, w64);
         if (L::D != 3) w64 = 0.0;
       } else {
-        float fg[L::Q];
-#pragma unroll
-        for (int p = 0; p < L::Q; ++p) fg[p] = ldf<L, S>(a, sb, p);
         float px, py, pz;
         load_force<L, float>(a, a.force_prev, g[0], g[1], gk, px, py, pz);
-        moments32<L>(fg, px, py, pz, dr32, u32, v32, w32);
+        moments32<L>(reinterpret_cast<const float *>(fs), px, py, pz, dr32, u32, v32, w32);
       }
     }
 #pragma unroll
     for (int q = 1; q < L::Q; ++q) {
-      const int di = g[0] + L::cx(q), dj = g[1] + L::cy(q), dk = gk + L::cz(q);
-      if (!in_box(a.lo, a.hi, di, dj, dk)) continue;
-      const R fq = ldf<L, S>(a, sb, q);
+      if (!enters(q)) continue;
+      const R fq = fs[q];
       R val;
       if (mode == 0) {
         val = fq;
@@ -360,10 +378,10 @@ __device__ __noinline__ void ghost_push(const StepArgs &a, int64_t gid, int64_t 
           val = R(post32<L>(q, float(fq), col32_setup<L>(dr32, u32, v32, w32, a.om32, a.omh32,
                                                          float(gFx), float(gFy), float(gFz))));
       }
-      Store<S>::store(fo + fidx(a, di, dj, dk) + q * a.fs2, val, sfac<L, S>(a, q));
+      Store<S>::store(fo + fidx(a, g[0] + L::cx(q), g[1] + L::cy(q), gk + L::cz(q)) + q * a.fs2, val,
+                      sfac<L, S>(a, q));
     }
   }
-  }  // slab
 }
 
 // ---------------------------------------------------------------------------
@@ -604,9 +622,9 @@ __device__ __forceinline__ void cell_fast(const StepArgs &a, int i, int j, int k
 template <class L, int S>
 __global__ void __launch_bounds__(256, StepOcc<L, S>::value) k_step(const __grid_constant__ StepArgs a) {
   if ((int)blockIdx.z < a.ghost_slices) {
-    const int64_t blk = blockIdx.x + (int64_t)gridDim.x * (blockIdx.y + (int64_t)gridDim.y * blockIdx.z);
+    const uint32_t blk = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
     ghost_push<L, S>(a, blk * blockDim.x + threadIdx.x,
-                     (int64_t)a.ghost_slices * gridDim.x * gridDim.y * blockDim.x);
+                     (uint32_t)a.ghost_slices * gridDim.x * gridDim.y * blockDim.x);
     return;
   }
   const int i0 = a.rlo[0] + blockIdx.x * blockDim.x;
@@ -666,8 +684,8 @@ __global__ void __launch_bounds__(256, BatchOcc<L, S>::value)
       cur = tl.c;
     }
     if (tl.i0 < 0) {
-      ghost_push<L, S>(sa, (int64_t)(-1 - tl.i0) * blockDim.x + threadIdx.x,
-                       (int64_t)tl.j * blockDim.x);
+      ghost_push<L, S>(sa, (uint32_t)(-1 - tl.i0) * blockDim.x + threadIdx.x,
+                       (uint32_t)tl.j * blockDim.x);
       continue;
     }
     // lean row segments as in k_step (a skip box, which single-level cases
@@ -983,6 +1001,31 @@ static int launch_band_macro_list(ilbm_ctx *ctx, const StepArgs &a, const int *b
 // ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
+// The ghost shell's sequence (ghost_push): slab d's cells lie outside the box
+// in dimension d (two faces), inside it in the active dimensions below d, on
+// the grown range of the other dimensions.  Inactive dimensions (periodic
+// with self-filled ghosts) have no slab.
+static int ghost_offsets(int D, StepArgs &a) {
+  int64_t off = 0;
+  for (int d = 0; d < 3; ++d) {
+    a.goff[d] = (uint32_t)off;
+    if (d >= D || (a.self_fill && a.periodic[d])) continue;
+    int64_t s = 2;
+    for (int e = 0; e < D; ++e)
+      if (e != d) {
+        const bool inner = e < d && !(a.self_fill && a.periodic[e]);
+        s *= (int64_t)(a.hi[e] - a.lo[e] + 1) + (inner ? 0 : 2);
+      }
+    off += s;
+    if (off > INT32_MAX) {
+      set_error("box too large: its ghost shell has 2^31 cells or more");
+      return ILBM_ERR_RANGE;
+    }
+  }
+  a.goff[3] = (uint32_t)off;
+  return ILBM_OK;
+}
+
 static int fill_args(const ilbm_ctx *ctx, const ilbm_box &b, const ilbm_level_params *p,
                      StepArgs &a) {
   std::memset(&a, 0, sizeof(a));
@@ -1061,6 +1104,8 @@ static int fill_args(const ilbm_ctx *ctx, const ilbm_box &b, const ilbm_level_pa
       a.act_lo[d] = (a.lo[d] == a.dlo[d]) && plo;
       a.act_hi[d] = (a.hi[d] == a.dhi[d]) && phi;
     }
+    int rc = ghost_offsets(D, a);
+    if (rc) return rc;
     if (p->ghost_mode == ILBM_GHOST_CALLER) {
       if (p->nlevel_boxes > kMaxLevelBoxes) {
         set_error("level has more boxes than one call supports (64); split the call");
@@ -1074,21 +1119,6 @@ static int fill_args(const ilbm_ctx *ctx, const ilbm_box &b, const ilbm_level_pa
     a.f16_scale = 1024.0f;
   }
   return ILBM_OK;
-}
-
-// ghost cells whose populations ghost_push delivers (0 when every face is a
-// self-filled periodic one)
-template <class L>
-static int64_t ghost_work(const StepArgs &a) {
-  int64_t n = 0;
-  for (int d = 0; d < L::D; ++d) {
-    if (a.self_fill && a.periodic[d]) continue;
-    int64_t s = 1;
-    for (int e = 0; e < L::D; ++e)
-      if (e != d) s *= (a.hi[e] - a.lo[e] + 3);
-    n += 2 * s;
-  }
-  return n;
 }
 
 // k_step over [rlo, rhi] (minus the skip box), with the ghost shell push in
@@ -1105,7 +1135,7 @@ static void launch_cells(ilbm_ctx *ctx, const StepArgs &a_in, cudaStream_t st, b
   if (with_ghosts) {
     // about one ghost cell per thread
     const int64_t per_slice = (int64_t)gx * ny * bx;
-    const int64_t w = ghost_work<L>(a);
+    const int64_t w = a.goff[3];
     if (w > 0) a.ghost_slices = (int)std::min<int64_t>(64, (w + per_slice - 1) / per_slice);
   }
   dim3 grid(gx, ny, nz + a.ghost_slices);
@@ -1301,18 +1331,9 @@ int batch_case_args(const ilbm_ctx *ctx, const ilbm_box &b, const ilbm_level_par
   return ILBM_OK;
 }
 
-// ghost-push chunks of w threads for one case (each thread takes at most one
-// ghost cell per slab); 0 when every face is a self-filled periodic one
-int batch_ghost_chunks(const ilbm_ctx *ctx, const StepArgs &a, int w) {
-  int64_t maxslab = 0;
-  for (int d = 0; d < ctx->dim; ++d) {
-    if (a.self_fill && a.periodic[d]) continue;
-    int64_t s = 1;
-    for (int e = 0; e < ctx->dim; ++e)
-      if (e != d) s *= (a.hi[e] - a.lo[e] + 3);
-    maxslab = std::max(maxslab, s);
-  }
-  return (int)((maxslab + w - 1) / w);
+// ghost-push chunks of w threads for one case (one ghost cell per thread); 0 when every face is a self-filled periodic one
+int batch_ghost_chunks(const ilbm_ctx *, const StepArgs &a, int w) {
+  return (int)(((int64_t)a.goff[3] + w - 1) / w);
 }
 
 template <class L, int S>

@@ -41,6 +41,9 @@ struct StepArgs {
   int slo[3], shi[3];
   int use_skip;
   int ghost_slices;          // leading z-slices of the k_step grid that run ghost_push
+  // the ghost shell in one sequence: first index of each dimension's slab,
+  // and the total (ghost_push)
+  uint32_t goff[4];
   int act_lo[3], act_hi[3];  // face returns outgoing populations (wrap / reflect)
   int nlb;
   int lb[kMaxLevelBoxes][6];
