@@ -53,7 +53,7 @@ def build(force: bool = False, verbose: bool = False, extra: list[str] | None = 
         if force or not o.exists() or o.stat().st_mtime < max(s.stat().st_mtime, dep_mtime):
             jobs.append((s, o))
     if jobs:
-        with cf.ThreadPoolExecutor(max_workers=min(8, len(jobs))) as ex:
+        with cf.ThreadPoolExecutor(max_workers=min(12, len(jobs))) as ex:
             futs = [ex.submit(_compile, s, o, extra) for s, o in jobs]
             for f in futs:
                 f.result()

@@ -46,6 +46,7 @@ struct ilbm_batch {
   StepArgs *d_args = nullptr;  // [2][ncase]
   StepTile *d_tiles = nullptr;
   int ntiles = 0, blocks = 0;
+  int V = 1;  // cells per thread of the level step
   IBBatch *ibb = nullptr;
   cudaGraphExec_t gexec[2] = {nullptr, nullptr};
   int64_t graph_launches[2] = {0, 0};
@@ -175,7 +176,8 @@ int build(ilbm_batch *b) {
   // finished its steps take the other cases' segments.
   const int W = b->tile_w;
   int per_sm = 0;
-  if ((rc = batch_step_occupancy(ctx, W, &per_sm))) return rc;
+  if ((rc = batch_plan(ctx, args.data(), 2 * nc, &b->V))) return rc;
+  if ((rc = batch_step_occupancy(ctx, b->V, W, &per_sm))) return rc;
   if (per_sm < 1) {
     set_error("batch: the level-step kernel does not fit this tile width");
     return ILBM_ERR_UNSUPPORTED;
@@ -184,15 +186,15 @@ int build(ilbm_batch *b) {
   std::vector<StepTile> tiles;
   for (int c = 0; c < nc; ++c) {
     const int nch = batch_ghost_chunks(ctx, args[c], W);
-    for (int ch = 0; ch < nch; ++ch) tiles.push_back(StepTile{c, -1 - ch, nch, 0});
+    for (int ch = 0; ch < nch; ++ch)
+      tiles.push_back(StepTile{c, (uint32_t)ch * (uint32_t)W, (uint32_t)nch * (uint32_t)W});
   }
   std::vector<std::vector<StepTile>> rows(nc);
   int64_t nrow = 0;
   for (int c = 0; c < nc; ++c) {
     const StepArgs &a = args[c];
-    for (int k = a.lo[2]; k <= a.hi[2]; ++k)
-      for (int j = a.lo[1]; j <= a.hi[1]; ++j)
-        for (int i0 = a.lo[0]; i0 <= a.hi[0]; i0 += W) rows[c].push_back(StepTile{c, i0, j, k});
+    const uint32_t per = batch_per_block(b->V, W);
+    for (uint32_t v = 0; v < a.nvec; v += per) rows[c].push_back(StepTile{c, v, 0});
     nrow += (int64_t)rows[c].size();
   }
   const int G = (int)std::max<int64_t>(1, std::min<int64_t>(nrow + (int64_t)tiles.size(),
@@ -217,7 +219,7 @@ int build(ilbm_batch *b) {
     int64_t rounds = 0;
     for (int c = 0; c < nc; ++c)
       rounds = std::max<int64_t>(rounds, ((int64_t)rows[c].size() + nb[c] - 1) / nb[c]);
-    while (tiles.size() % G) tiles.push_back(StepTile{-1, 0, 0, 0});
+    while (tiles.size() % G) tiles.push_back(StepTile{-1, 0, 0});
     std::vector<int> owner(G), first(nc + 1, 0);
     for (int c = 0; c < nc; ++c) first[c + 1] = first[c] + nb[c];
     for (int c = 0; c < nc; ++c)
@@ -226,7 +228,7 @@ int build(ilbm_batch *b) {
       for (int s = 0; s < G; ++s) {
         const int c = owner[s];
         const int64_t i = r * nb[c] + (s - first[c]);
-        tiles.push_back(i < (int64_t)rows[c].size() ? rows[c][(size_t)i] : StepTile{-1, 0, 0, 0});
+        tiles.push_back(i < (int64_t)rows[c].size() ? rows[c][(size_t)i] : StepTile{-1, 0, 0});
       }
   } else {
     for (int c = 0; c < nc; ++c) tiles.insert(tiles.end(), rows[c].begin(), rows[c].end());
@@ -261,7 +263,7 @@ int step_slot(ilbm_batch *b, int slot) {
   const StepArgs *a = b->d_args + (size_t)slot * nc;
   int rc = ib_batch_forcing(b->ibb, a, b->ctx->stream);
   if (rc) return rc;
-  if ((rc = batch_step_launch(b->ctx, a, b->d_tiles, b->ntiles, b->tile_w, b->blocks,
+  if ((rc = batch_step_launch(b->ctx, a, b->d_tiles, b->ntiles, b->V, b->tile_w, b->blocks,
                               ib_batch_steps(b->ibb), ib_batch_limits(b->ibb), b->ctx->stream)))
     return rc;
   return ib_batch_record(b->ibb, a, b->ctx->stream);
@@ -471,7 +473,8 @@ int ilbm_batch_tune(ilbm_batch *b, int trial_steps, int *tile_w, int *ctas_per_s
   int bw = b->tile_w, bc = b->ctas_per_sm;
   for (int w : {64, 128, 256}) {
     int per_sm = 0;
-    int rc = batch_step_occupancy(b->ctx, w, &per_sm);
+    int rc = build(b);  // (the vector width of the cases at hand)
+    if (!rc) rc = batch_step_occupancy(b->ctx, b->V, w, &per_sm);
     if (rc) return rc;
     for (int cps = per_sm; cps >= 1 && cps >= per_sm - 2; --cps) {
       if ((rc = ilbm_batch_set_tiles(b, w, cps))) return rc;

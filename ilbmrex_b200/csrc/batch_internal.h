@@ -24,16 +24,20 @@ int batch_case_args(const ilbm_ctx *ctx, const ilbm_box &b, const ilbm_level_par
                     StepArgs *out);
 // ghost-push chunks of w threads one case needs
 int batch_ghost_chunks(const ilbm_ctx *ctx, const StepArgs &a, int w);
+// the vector sequence of every case's cells (V cells per vector, the same for all)
+int batch_plan(const ilbm_ctx *ctx, StepArgs *args, int n, int *V);
+// vectors of a case that a tile of w threads takes
+uint32_t batch_per_block(int V, int w);
 // k_step_batch over a tile table (w threads per block, `blocks` persistent
 // blocks); cases with steps[c] >= limit[c] are skipped
 int batch_step_launch(ilbm_ctx *ctx, const StepArgs *d_args, const StepTile *d_tiles, int ntiles,
-                      int w, int blocks, const int *steps, const int *limit, cudaStream_t st);
+                      int V, int w, int blocks, const int *steps, const int *limit, cudaStream_t st);
 // band macro of every case's body over its band tiles (same skipping)
 int batch_band_macro_launch(ilbm_ctx *ctx, const StepArgs *d_args, const BandDesc *d_bands,
                             const ItemRef *d_tiles, int ntiles, const int *steps, const int *limit,
                             cudaStream_t st);
 // resident blocks of w threads per SM of k_step_batch
-int batch_step_occupancy(const ilbm_ctx *ctx, int w, int *per_sm);
+int batch_step_occupancy(const ilbm_ctx *ctx, int V, int w, int *per_sm);
 
 // ---- forces.cu ------------------------------------------------------------
 // the Eulerian force sum of ilbm_force_integrals enqueued on ctx->stream; the

@@ -174,7 +174,7 @@ __device__ __forceinline__ double collide64_one(int q, double f, double feq, dou
 
 // ---------------------------------------------------------------------------
 // Storage forms.  load() returns the working value (f for F64, g = f - w for
-// the shifted forms); store() converts it back.
+// the shifted forms); store() / pack() convert it back.
 // ---------------------------------------------------------------------------
 template <int S>
 struct Store;
@@ -187,6 +187,7 @@ struct Store<ILBM_STORAGE_F64> {
   __device__ static __forceinline__ R load(const T *p, float) { return *p; }
   __device__ static __forceinline__ R cvt(T v, float) { return v; }
   __device__ static __forceinline__ void store(T *p, R v, float) { *p = v; }
+  __device__ static __forceinline__ T pack(R v, float) { return v; }
 };
 
 template <>
@@ -197,6 +198,7 @@ struct Store<ILBM_STORAGE_F32_SHIFT> {
   __device__ static __forceinline__ R load(const T *p, float) { return __ldg(p); }
   __device__ static __forceinline__ R cvt(T v, float) { return v; }
   __device__ static __forceinline__ void store(T *p, R v, float) { *p = v; }
+  __device__ static __forceinline__ T pack(R v, float) { return v; }
 };
 
 template <>
@@ -208,6 +210,8 @@ struct Store<ILBM_STORAGE_F16_SCALED> {
   __device__ static __forceinline__ R load(const T *p, float s) { return __half2float(*p) * s; }
   __device__ static __forceinline__ R cvt(T v, float s) { return __half2float(v) * s; }
   __device__ static __forceinline__ void store(T *p, R v, float s) { *p = __float2half_rn(v / s); }
+  // si: the inverse factor scale / w_q
+  __device__ static __forceinline__ T pack(R v, float si) { return __float2half_rn(v * si); }
 };
 
 // rho, u of a cell from its populations and the previous force

@@ -29,6 +29,8 @@
 
 #include "ilbm_common.cuh"
 #include "step_args.cuh"
+#include "step_device.cuh"
+#include "step_launch.h"
 
 namespace ilbm {
 
@@ -38,670 +40,6 @@ const char *get_error() { return g_err.c_str(); }
 int cuda_fail(cudaError_t e, const char *what) {
   set_error(std::string(what) + ": " + cudaGetErrorString(e));
   return ILBM_ERR_CUDA;
-}
-
-
-__device__ __forceinline__ int64_t fidx(const StepArgs &a, int i, int j, int k) {
-  return (int64_t)(i - a.fgl[0]) + (int64_t)(j - a.fgl[1]) * a.fs0 +
-         (int64_t)(k - a.fgl[2]) * a.fs1;
-}
-__device__ __forceinline__ int64_t midx(const StepArgs &a, int i, int j, int k) {
-  return (int64_t)(i - a.mgl[0]) + (int64_t)(j - a.mgl[1]) * a.ms0 +
-         (int64_t)(k - a.mgl[2]) * a.ms1;
-}
-
-template <class L>
-__device__ __forceinline__ bool in_domain(const StepArgs &a, int i, int j, int k) {
-  if (i < a.dlo[0] || i > a.dhi[0] || j < a.dlo[1] || j > a.dhi[1]) return false;
-  if (L::D == 3 && (k < a.dlo[2] || k > a.dhi[2])) return false;
-  return true;
-}
-
-// per-direction storage factor for the F16 form: w_q / scale
-template <class L, int S>
-__device__ __forceinline__ float sfac(const StepArgs &a, int q) {
-  if (S == ILBM_STORAGE_F16_SCALED) return float(L::w(q)) / a.f16_scale;
-  return 1.0f;
-}
-
-template <class L, int S>
-__device__ __forceinline__ typename Store<S>::R ldf(const StepArgs &a, int64_t base, int q) {
-  using T = typename Store<S>::T;
-  return Store<S>::load(static_cast<const T *>(a.f_in) + base + q * a.fs2, sfac<L, S>(a, q));
-}
-
-template <class R>
-__device__ __forceinline__ R ldm(const void *p, int64_t idx) {
-  return static_cast<const R *>(p)[idx];
-}
-
-// force at a cell (F^n or F^{n-1}); zero outside the force region
-template <class L, class R>
-__device__ __forceinline__ void load_force(const StepArgs &a, const void *F, int i, int j,
-                                           int k, R &fx, R &fy, R &fz) {
-  if (F == nullptr) {
-    if (a.use_uniform) {
-      fx = R(a.uf[0]);
-      fy = R(a.uf[1]);
-      fz = R(a.uf[2]);
-    } else {
-      fx = fy = fz = R(0);
-    }
-    return;
-  }
-  if (i < a.flo[0] || i > a.fhi[0] || j < a.flo[1] || j > a.fhi[1] ||
-      (L::D == 3 && (k < a.flo[2] || k > a.fhi[2]))) {
-    fx = fy = fz = R(0);
-    return;
-  }
-  const int64_t m = midx(a, i, j, k);
-  fx = ldm<R>(F, m);
-  fy = ldm<R>(F, m + a.ms2);
-  fz = (L::D == 3) ? ldm<R>(F, m + 2 * a.ms2) : R(0);
-}
-
-// ---------------------------------------------------------------------------
-// Ghost synthesis (pre-collision values of physical-boundary ghosts), with the
-// FillPatch semantics the reference relies on: periodic images first, then per
-// ghost cell AMReX's foextrap fill followed by mesoscopicBcFill
-// (Source/BC/bc_fill.H:303-347: user_2 face mirror > user_1 copy > ext_dir
-// non-equilibrium extrapolation, mirror = nearest domain cell).
-// ---------------------------------------------------------------------------
-template <class L>
-__device__ __forceinline__ bool first_face(const StepArgs &a, const int *g, int type, int &bd,
-                                           int &lo_side) {
-#pragma unroll
-  for (int d = 0; d < L::D; ++d) {
-    if (g[d] < a.dlo[d] && a.bclo[d] == type) { bd = d; lo_side = 1; return true; }
-    if (g[d] > a.dhi[d] && a.bchi[d] == type) { bd = d; lo_side = 0; return true; }
-  }
-  return false;
-}
-
-// Resolve a ghost cell to either a source cell in the domain (copy) or a
-// boundary formula on a mirror cell.  kind: 0 copy src, 1 user_1 copy of
-// mirror, 2 ext_dir NEQ, 3 user_2 face-mirror NEQ.
-template <class L>
-__device__ __forceinline__ int ghost_rule(const StepArgs &a, const int *g, int *src, int &bd,
-                                          int &lo_side) {
-  int cur[3] = {g[0], g[1], g[2]};
-  for (int it = 0; it < 4; ++it) {
-    bool inside = true, wrappable = true;
-#pragma unroll
-    for (int d = 0; d < L::D; ++d) {
-      const bool out = cur[d] < a.dlo[d] || cur[d] > a.dhi[d];
-      if (out) {
-        inside = false;
-        if (!a.periodic[d]) wrappable = false;
-      }
-    }
-    if (inside || wrappable) {
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        int c = cur[d];
-        if (d < L::D && a.periodic[d]) {
-          const int n = a.dhi[d] - a.dlo[d] + 1;
-          while (c < a.dlo[d]) c += n;  // a ghost lies a cell or two outside
-          while (c > a.dhi[d]) c -= n;
-        }
-        src[d] = c;
-      }
-      return 0;
-    }
-    if (it == 0) {
-      int m[3] = {cur[0], cur[1], cur[2]};
-#pragma unroll
-      for (int d = 0; d < L::D; ++d) m[d] = min(max(cur[d], a.dlo[d]), a.dhi[d]);
-      if (first_face<L>(a, cur, ILBM_BC_USER_2, bd, lo_side)) { src[0] = m[0]; src[1] = m[1]; src[2] = m[2]; return 3; }
-      if (first_face<L>(a, cur, ILBM_BC_USER_1, bd, lo_side)) { src[0] = m[0]; src[1] = m[1]; src[2] = m[2]; return 1; }
-      if (first_face<L>(a, cur, ILBM_BC_EXT_DIR, bd, lo_side)) { src[0] = m[0]; src[1] = m[1]; src[2] = m[2]; return 2; }
-    }
-    // foextrap: the last dimension with a foextrap face wins (FilccCell order)
-    int dsel = -1;
-#pragma unroll
-    for (int d = 0; d < L::D; ++d) {
-      if (cur[d] < a.dlo[d] && a.bclo[d] == ILBM_BC_FOEXTRAP) dsel = d;
-      else if (cur[d] > a.dhi[d] && a.bchi[d] == ILBM_BC_FOEXTRAP) dsel = d;
-    }
-    if (dsel < 0) break;
-#pragma unroll
-    for (int d = 0; d < L::D; ++d)  // (constant subscripts: cur stays in registers)
-      if (d == dsel) cur[d] = (cur[d] < a.dlo[d]) ? a.dlo[d] : a.dhi[d];
-  }
-  src[0] = min(max(g[0], a.dlo[0]), a.dhi[0]);
-  src[1] = min(max(g[1], a.dlo[1]), a.dhi[1]);
-  src[2] = (L::D == 3) ? min(max(g[2], a.dlo[2]), a.dhi[2]) : 0;
-  return 0;
-}
-
-// Populations that enter the box from its layer-1 ghost shell are pushed here,
-// one thread per ghost cell: the pre-collision boundary value (self-fill: the
-// FillPatch rules above on f^n of the domain; caller-filled: the ghost value
-// as given), or, for a ghost covered by another box of the level, that cell's
-// post-collision value.  Ghosts that are periodic images (self-fill) and
-// halfway bounce-back ghosts are left to the owning cells' push.  A ghost cell
-// is owned by the slab of its lowest dimension outside the box (periodic
-// dimensions excluded in self-fill mode, whose slabs do not exist), so the
-// shell is one sequence of cells: slab d holds the cells outside the box in
-// dimension d, inside it in the active dimensions below d, and on the grown
-// range of the others (StepArgs::goff, filled by ghost_offsets).
-// The work runs in the leading blocks of the k_step launch (it writes only
-// slots that no cell's push writes, and reads only f^n), so its strided
-// accesses overlap the main stream instead of preceding it.  It is bound by
-// latency: one thread's chain is one ghost's index, its loads in flight
-// together, and its stores.  A thread that walked the 2 D slabs one after
-// another, each with 64-bit index divisions and a load per direction before
-// its store, was the tail of every small launch: a 50 x 50 x 45 FP64 box with
-// covered ghosts took 61 us against 5 us of traffic, and twelve of them 774 us
-// against 320 us with one ghost per thread; the three-level 1024 x 512
-// cylinder 213 -> 182 us per coarse step.  Loading only the entering
-// directions of a copied ghost matters too: all 19 made the two-level sphere
-// 1.3% slower than before instead of 1.3% faster.
-template <class L>
-__device__ __forceinline__ bool ghost_active(const StepArgs &a, int d) {
-  return !(a.self_fill && a.periodic[d]);
-}
-
-template <class L, int S>
-__device__ __noinline__ void ghost_push(const StepArgs &a, uint32_t gid, uint32_t gstride) {
-  using T = typename Store<S>::T;
-  using R = typename Store<S>::R;
-  T *fo = static_cast<T *>(a.f_out);
-  const uint32_t total = a.goff[3];
-  for (uint32_t t = gid; t < total; t += gstride) {
-    const int d = (int)(t >= a.goff[1]) + (int)(L::D == 3 && t >= a.goff[2]);
-    uint32_t r = t - (d == 0 ? 0u : (d == 1 ? a.goff[1] : a.goff[2]));
-    int g[3] = {0, 0, 0};
-#pragma unroll
-    for (int e = 0; e < L::D; ++e) {
-      const bool inner = e < d && ghost_active<L>(a, e);
-      const uint32_t n = (uint32_t)(a.hi[e] - a.lo[e] + 1);
-      const uint32_t ext = (e == d) ? 2u : (inner ? n : n + 2u);
-      const uint32_t c = (e == L::D - 1) ? r : r % ext;
-      r /= ext;
-      g[e] = (e == d) ? (c ? a.hi[e] + 1 : a.lo[e] - 1) : a.lo[e] + (int)c - (inner ? 0 : 1);
-    }
-    // classify the ghost against the domain
-    bool phys = false, pure_u1 = true;
-#pragma unroll
-    for (int e = 0; e < L::D; ++e) {
-      int sd = 0;
-      if (g[e] < a.dlo[e]) sd = -1;
-      else if (g[e] > a.dhi[e]) sd = 1;
-      if (sd == 0) continue;
-      if (a.periodic[e]) {
-        pure_u1 = false;
-      } else {
-        phys = true;
-        if ((sd < 0 ? a.bclo[e] : a.bchi[e]) != ILBM_BC_USER_1) pure_u1 = false;
-      }
-    }
-    if (a.self_fill && !phys) continue;  // periodic image: the wrapping push delivers it
-    if (phys && pure_u1) continue;       // halfway bounce-back: reflected by the cell
-    const int gk = (L::D == 3) ? g[2] : 0;
-    // source of the ghost's populations
-    int mode;  // 0 copy from src (raw), 1 NEQ boundary formula on src, 2 collide the ghost
-    int src[3] = {g[0], g[1], gk}, bd = 0, lo_side = 1, kind = 0;
-    if (phys && a.self_fill) {
-      kind = ghost_rule<L>(a, g, src, bd, lo_side);
-      mode = (kind <= 1) ? 0 : 1;
-    } else if (phys) {
-      mode = 0;  // caller-filled physical ghost, as given
-    } else {
-      int gw[3] = {g[0], g[1], gk};
-#pragma unroll
-      for (int e = 0; e < L::D; ++e)
-        if (a.periodic[e]) {
-          const int nn = a.dhi[e] - a.dlo[e] + 1;
-          while (gw[e] < a.dlo[e]) gw[e] += nn;
-          while (gw[e] > a.dhi[e]) gw[e] -= nn;
-        }
-      bool covered = false;
-      for (int b = 0; b < a.nlb && !covered; ++b)
-        covered = gw[0] >= a.lb[b][0] && gw[0] <= a.lb[b][3] && gw[1] >= a.lb[b][1] &&
-                  gw[1] <= a.lb[b][4] && (L::D == 2 || (gw[2] >= a.lb[b][2] && gw[2] <= a.lb[b][5]));
-      mode = covered ? 2 : 0;  // not covered: coarse-fine ghost, as given
-    }
-    const int64_t sb = fidx(a, src[0], src[1], L::D == 3 ? src[2] : 0);
-    // the directions that enter the box, and the loads the ghost needs (those
-    // directions; all of them where moments are formed), in flight together
-    bool into[3][3];
-#pragma unroll
-    for (int e = 0; e < 3; ++e)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const int x = ((e == 2) ? gk : g[e]) + c - 1;
-        into[e][c] = x >= a.lo[e] && x <= a.hi[e];
-      }
-    auto enters = [&](int q) {
-      return into[0][L::cx(q) + 1] && into[1][L::cy(q) + 1] && into[2][L::cz(q) + 1];
-    };
-    R fs[L::Q];
-#pragma unroll
-    for (int q = 0; q < L::Q; ++q) fs[q] = (mode != 0 || enters(q)) ? ldf<L, S>(a, sb, q) : R(0);
-    // per-ghost state for the NEQ formula / the collision
-    double r64 = 0, u64 = 0, v64 = 0, w64 = 0, rt64 = 0, ut64 = 0, vt64 = 0, wt64 = 0;
-    float dr32 = 0, u32 = 0, v32 = 0, w32 = 0, drt32 = 0, ut32 = 0, vt32 = 0, wt32 = 0;
-    R gFx = R(0), gFy = R(0), gFz = R(0);
-    bool ghf = false;
-    if (mode == 1) {
-      // applyExtDirMesoscopic / applyFaceMirroredMesoscopic, bc_fill.H:159-261
-      const double *bv = lo_side ? a.bvlo[bd] : a.bvhi[bd];
-      if (S == ILBM_STORAGE_F64) {
-        double rhonp = 0.0, unp = 0.0, vnp = 0.0, wnp = 0.0;
-#pragma unroll
-        for (int p = 0; p < L::Q; ++p) {
-          const double fp = fs[p];
-          rhonp = X::add(rhonp, fp);
-          unp = X::add(unp, X::mul(double(L::cx(p)), fp));
-          vnp = X::add(vnp, X::mul(double(L::cy(p)), fp));
-          wnp = X::add(wnp, X::mul(double(L::cz(p)), fp));
-        }
-        rhonp = fmax(rhonp, 1.0e-20);
-        r64 = rhonp;
-        u64 = X::div(unp, rhonp);
-        v64 = X::div(vnp, rhonp);
-        w64 = X::div(wnp, rhonp);
-        rt64 = bv[0]; ut64 = bv[1]; vt64 = bv[2]; wt64 = bv[3];
-        if (kind == 3) {
-          rt64 = fmax(1.0e-20, X::sub(X::mul(2.0, bv[0]), r64));
-          ut64 = X::sub(X::mul(2.0, bv[1]), u64);
-          vt64 = X::sub(X::mul(2.0, bv[2]), v64);
-          wt64 = X::sub(X::mul(2.0, bv[3]), w64);
-        }
-      } else {
-        float rr = 0.f, m1 = 0.f, m2 = 0.f, m3 = 0.f;
-#pragma unroll
-        for (int p = 0; p < L::Q; ++p) {
-          const float gp = fs[p];
-          rr += gp;
-          if (L::cx(p)) m1 += float(L::cx(p)) * gp;
-          if (L::cy(p)) m2 += float(L::cy(p)) * gp;
-          if (L::cz(p)) m3 += float(L::cz(p)) * gp;
-        }
-        const float rho = fmaxf(1.0f + rr, 1.0e-20f);
-        dr32 = rho - 1.0f;
-        u32 = m1 / rho; v32 = m2 / rho; w32 = m3 / rho;
-        drt32 = float(bv[0]) - 1.0f; ut32 = float(bv[1]); vt32 = float(bv[2]); wt32 = float(bv[3]);
-        if (kind == 3) {
-          drt32 = fmaxf(1.0e-20f, 2.0f * float(bv[0]) - rho) - 1.0f;
-          ut32 = 2.0f * float(bv[1]) - u32;
-          vt32 = 2.0f * float(bv[2]) - v32;
-          wt32 = 2.0f * float(bv[3]) - w32;
-        }
-      }
-    } else if (mode == 2) {
-      load_force<L, R>(a, a.force, g[0], g[1], gk, gFx, gFy, gFz);
-      ghf = !(gFx == R(0) && gFy == R(0) && gFz == R(0));
-      if (stored_macro_at(a, g[0], g[1], gk)) {
-        const int64_t m = midx(a, g[0], g[1], gk);
-        if (S == ILBM_STORAGE_F64) {
-          r64 = ldm<double>(a.macro_in, m);
-          u64 = ldm<double>(a.macro_in, m + a.ms2);
-          v64 = ldm<double>(a.macro_in, m + 2 * a.ms2);
-          w64 = (L::D == 3) ? ldm<double>(a.macro_in, m + 3 * a.ms2) : 0.0;
-        } else {
-          dr32 = ldm<float>(a.macro_in, m) - 1.0f;
-          u32 = ldm<float>(a.macro_in, m + a.ms2);
-          v32 = ldm<float>(a.macro_in, m + 2 * a.ms2);
-          w32 = (L::D == 3) ? ldm<float>(a.macro_in, m + 3 * a.ms2) : 0.0f;
-        }
-      } else if (S == ILBM_STORAGE_F64) {
-        double px, py, pz;
-        load_force<L, double>(a, a.force_prev, g[0], g[1], gk, px, py, pz);
-        moments64<L>(reinterpret_cast<const double *>(fs), px, py, pz, r64, u64, v64, w64);
-        if (L::D != 3) w64 = 0.0;
-      } else {
-        float px, py, pz;
-        load_force<L, float>(a, a.force_prev, g[0], g[1], gk, px, py, pz);
-        moments32<L>(reinterpret_cast<const float *>(fs), px, py, pz, dr32, u32, v32, w32);
-      }
-    }
-#pragma unroll
-    for (int q = 1; q < L::Q; ++q) {
-      if (!enters(q)) continue;
-      const R fq = fs[q];
-      R val;
-      if (mode == 0) {
-        val = fq;
-      } else if (mode == 1) {
-        if (S == ILBM_STORAGE_F64)
-          val = R(X::add(feq64_3<L>(q, rt64, ut64, vt64, wt64),
-                         X::sub(double(fq), feq64_3<L>(q, r64, u64, v64, w64))));
-        else
-          val = R(feqs<L>(q, drt32, ut32, vt32, wt32) + (float(fq) - feqs<L>(q, dr32, u32, v32, w32)));
-      } else {
-        if (S == ILBM_STORAGE_F64)
-          val = R(collide64_one<L>(q, double(fq), feq64<L>(q, r64, u64, v64, w64), a.tau, u64, v64,
-                                   w64, double(gFx), double(gFy), double(gFz), ghf));
-        else
-          val = R(post32<L>(q, float(fq), col32_setup<L>(dr32, u32, v32, w32, a.om32, a.omh32,
-                                                         float(gFx), float(gFy), float(gFz))));
-      }
-      Store<S>::store(fo + fidx(a, g[0] + L::cx(q), g[1] + L::cy(q), gk + L::cz(q)) + q * a.fs2, val,
-                      sfac<L, S>(a, q));
-    }
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Main fused kernel
-// ---------------------------------------------------------------------------
-// occupancy target: 4 resident blocks of 256 threads per SM for the 4-byte and
-// 2-byte storage forms of D2Q9/D3Q19 (<= 64 registers), 2 otherwise
-template <class L, int S>
-struct StepOcc {
-  static constexpr int value = (S != ILBM_STORAGE_F64 && L::Q <= 19) ? 4 : 2;
-};
-
-// One cell of the level step: load f^n, recover rho^n/u^n, collide, push.
-// `edge` selects the checked push plus the completion of ghost-sourced pulls;
-// interior cells take the unchecked path.
-template <class L, int S>
-__device__ __forceinline__ void cell_finish(const StepArgs &a, int i, int j, int k, bool edge,
-                                            typename Store<S>::R *f);
-
-template <class L, int S>
-__device__ __forceinline__ void cell_update(const StepArgs &a, int i, int j, int k, bool edge) {
-  using T = typename Store<S>::T;
-  using R = typename Store<S>::R;
-  const T *fin = static_cast<const T *>(a.f_in) + fidx(a, i, j, k);
-  R f[L::Q];
-#pragma unroll
-  for (int q = 0; q < L::Q; ++q) f[q] = Store<S>::load(fin + a.loff[q], sfac<L, S>(a, q));
-  cell_finish<L, S>(a, i, j, k, edge, f);
-}
-
-// The rest of a cell update once its populations f^n are in registers.
-template <class L, int S>
-__device__ __forceinline__ void cell_finish(const StepArgs &a, int i, int j, int k, bool edge,
-                                            typename Store<S>::R *f) {
-  using T = typename Store<S>::T;
-  using R = typename Store<S>::R;
-  const int64_t base = fidx(a, i, j, k);
-  R Fx, Fy, Fz;
-  load_force<L, R>(a, a.force, i, j, k, Fx, Fy, Fz);
-
-  // per-cell collision state: rho^n, u^n (stored or recovered) and F^n
-  double rho64 = 0, u64 = 0, v64 = 0, w64 = 0;
-  float drho32 = 0, u32 = 0, v32 = 0, w32 = 0;
-  const bool stored = stored_macro_at(a, i, j, k);
-  if (S == ILBM_STORAGE_F64) {
-    if (stored) {
-      const int64_t m = midx(a, i, j, k);
-      rho64 = ldm<double>(a.macro_in, m);
-      u64 = ldm<double>(a.macro_in, m + a.ms2);
-      v64 = ldm<double>(a.macro_in, m + 2 * a.ms2);
-      w64 = (L::D == 3) ? ldm<double>(a.macro_in, m + 3 * a.ms2) : 0.0;
-    } else {
-      double px, py, pz;
-      load_force<L, double>(a, a.force_prev, i, j, k, px, py, pz);
-      moments64<L>(reinterpret_cast<double *>(f), px, py, pz, rho64, u64, v64, w64);
-      if (L::D != 3) w64 = 0.0;
-    }
-  } else {
-    if (stored) {
-      const int64_t m = midx(a, i, j, k);
-      drho32 = ldm<float>(a.macro_in, m) - 1.0f;
-      u32 = ldm<float>(a.macro_in, m + a.ms2);
-      v32 = ldm<float>(a.macro_in, m + 2 * a.ms2);
-      w32 = (L::D == 3) ? ldm<float>(a.macro_in, m + 3 * a.ms2) : 0.0f;
-    } else {
-      float px, py, pz;
-      load_force<L, float>(a, a.force_prev, i, j, k, px, py, pz);
-      moments32<L>(reinterpret_cast<float *>(f), px, py, pz, drho32, u32, v32, w32);
-    }
-  }
-  // the Guo increment is skipped where F == 0 (collide_forced.H:81-83)
-  const bool hf = !(Fx == R(0) && Fy == R(0) && Fz == R(0));
-  const Col32 c32 = col32_setup<L>(drho32, u32, v32, w32, a.om32, a.omh32, float(Fx), float(Fy),
-                                   float(Fz));
-  auto post_v = [&](int q, R fq) -> R {
-    if (S == ILBM_STORAGE_F64) {
-      const double fe = feq64<L>(q, rho64, u64, v64, w64);
-      return R(collide64_one<L>(q, double(fq), fe, a.tau, u64, v64, w64, double(Fx),
-                                double(Fy), double(Fz), hf));
-    } else {
-      return R(post32<L>(q, float(fq), c32));
-    }
-  };
-
-  T *fo = static_cast<T *>(a.f_out);
-  T *fob = fo + base;
-  // Push: every thread, edge or not, stores f*(y,q) at y + c_q.  For an edge
-  // cell some of these land in the ghost layer of f_out, which is scratch
-  // (never read); they are fixed up below.
-#pragma unroll
-  for (int q = 0; q < L::Q; ++q) Store<S>::store(fob + a.doff[q], post_v(q, f[q]), sfac<L, S>(a, q));
-  if (!edge) return;
-  // Edge fix-up for destinations outside the box: periodic image (self-fill)
-  // -> wrapped push; halfway bounce-back wall -> reflected into this cell
-  // (f*(x,q) -> f_out(x, q_bar), AdvanceLBMAtLevel.cpp:272-373); anything
-  // else leaves the box (the populations entering from that ghost come from
-  // k_ghost_push).  The few populations involved are re-collided from a reload.
-  const T *fin_c = static_cast<const T *>(a.f_in) + base;
-#pragma unroll
-  for (int q = 1; q < L::Q; ++q) {
-    int di = i + L::cx(q), dj = j + L::cy(q), dk = k + L::cz(q);
-    if (in_box(a.lo, a.hi, di, dj, dk)) continue;
-    const int dd[3] = {di, dj, dk};
-    bool phys = false, pure_u1 = true;
-#pragma unroll
-    for (int e = 0; e < L::D; ++e) {
-      int sd = 0;
-      if (dd[e] < a.dlo[e]) sd = -1;
-      else if (dd[e] > a.dhi[e]) sd = 1;
-      if (sd == 0) continue;
-      if (a.periodic[e]) {
-        pure_u1 = false;
-      } else {
-        phys = true;
-        if ((sd < 0 ? a.bclo[e] : a.bchi[e]) != ILBM_BC_USER_1) pure_u1 = false;
-      }
-    }
-    T *dst;
-    if (phys) {
-      if (!pure_u1) continue;
-      dst = fob + a.loff[opposite<L>(q)];
-    } else if (a.self_fill) {
-      if (L::cx(q) != 0 && (di < a.dlo[0] || di > a.dhi[0])) di = (di < a.dlo[0]) ? a.dhi[0] : a.dlo[0];
-      if (L::cy(q) != 0 && (dj < a.dlo[1] || dj > a.dhi[1])) dj = (dj < a.dlo[1]) ? a.dhi[1] : a.dlo[1];
-      if (L::D == 3 && L::cz(q) != 0 && (dk < a.dlo[2] || dk > a.dhi[2]))
-        dk = (dk < a.dlo[2]) ? a.dhi[2] : a.dlo[2];
-      dst = fo + fidx(a, di, dj, dk) + (int64_t)q * a.fs2;
-    } else {
-      continue;  // another box: its ghost shell push delivers
-    }
-    const R fq = Store<S>::load(fin_c + a.loff[q], sfac<L, S>(a, q));
-    // (w_q = w_{q_bar}: the FP16 storage factor is the same for a reflection)
-    Store<S>::store(dst, post_v(q, fq), sfac<L, S>(a, q));
-  }
-}
-
-// Main kernel: one thread per cell of a row segment (rows on a box face run
-// the checked push as a whole; only the two x-edge cells of a row diverge).
-// the edge fix-up is needed only on faces whose outgoing populations come
-// back into the box (self-filled periodic: wrapped; user_1: reflected)
-template <class L>
-__device__ __forceinline__ bool needs_fixup(const StepArgs &a, int i, int j, int k) {
-  return (i == a.lo[0] && a.act_lo[0]) || (i == a.hi[0] && a.act_hi[0]) ||
-         (j == a.lo[1] && a.act_lo[1]) || (j == a.hi[1] && a.act_hi[1]) ||
-         (L::D == 3 && ((k == a.lo[2] && a.act_lo[2]) || (k == a.hi[2] && a.act_hi[2])));
-}
-
-// Row segments that need none of the per-cell tests of cell_update take a
-// lean path: no face of the segment returns outgoing populations (wrap /
-// reflect), no cell reads stored macro fields, none lies in the skip box,
-// and the force is of one kind over the whole segment.  The kind is the same
-// for every thread of a block (one block = one row segment), so the branch
-// does not diverge.
-enum SegKind { SEG_GENERAL = 0, SEG_SKIP = 1, SEG_ZERO = 2, SEG_UNIFORM = 3, SEG_ARRAYS = 4 };
-
-template <class L>
-__device__ __forceinline__ int seg_kind(const StepArgs &a, int i0, int i1, int j, int k) {
-  if (a.use_skip && j >= a.slo[1] && j <= a.shi[1] &&
-      (L::D == 2 || (k >= a.slo[2] && k <= a.shi[2]))) {
-    if (i0 >= a.slo[0] && i1 <= a.shi[0]) return SEG_SKIP;
-    if (!(i1 < a.slo[0] || i0 > a.shi[0])) return SEG_GENERAL;
-  }
-  if ((j == a.lo[1] && a.act_lo[1]) || (j == a.hi[1] && a.act_hi[1])) return SEG_GENERAL;
-  if (L::D == 3 && ((k == a.lo[2] && a.act_lo[2]) || (k == a.hi[2] && a.act_hi[2])))
-    return SEG_GENERAL;
-  if ((i0 == a.lo[0] && a.act_lo[0]) || (i1 == a.hi[0] && a.act_hi[0])) return SEG_GENERAL;
-  if (a.macro_in) {
-    if (!a.use_mbox) return SEG_GENERAL;
-    if (j >= a.mblo[1] && j <= a.mbhi[1] && k >= a.mblo[2] && k <= a.mbhi[2] &&
-        !(i1 < a.mblo[0] || i0 > a.mbhi[0]))
-      return SEG_GENERAL;
-  }
-  if (a.force == nullptr || a.force_prev == nullptr) {
-    if (a.force != nullptr || a.force_prev != nullptr) return SEG_GENERAL;
-    return a.use_uniform ? SEG_UNIFORM : SEG_ZERO;
-  }
-  // force arrays: zero outside [flo, fhi] (F^n and F^{n-1} alike)
-  if (j < a.flo[1] || j > a.fhi[1] || (L::D == 3 && (k < a.flo[2] || k > a.fhi[2])) ||
-      i1 < a.flo[0] || i0 > a.fhi[0])
-    return SEG_ZERO;
-  if (i0 >= a.flo[0] && i1 <= a.fhi[0]) return SEG_ARRAYS;
-  return SEG_GENERAL;
-}
-
-// One cell of a lean row segment: the same arithmetic as cell_update with
-// edge = false on rho^n, u^n recovered from f^n and F^{n-1}.
-template <class L, int S, int K>
-__device__ __forceinline__ void cell_fast(const StepArgs &a, int i, int j, int k) {
-  using T = typename Store<S>::T;
-  using R = typename Store<S>::R;
-  const int64_t base = fidx(a, i, j, k);
-  const T *fin = static_cast<const T *>(a.f_in) + base;
-  R f[L::Q];
-#pragma unroll
-  for (int q = 0; q < L::Q; ++q) f[q] = Store<S>::load(fin + a.loff[q], sfac<L, S>(a, q));
-  R Fx = R(0), Fy = R(0), Fz = R(0), px = R(0), py = R(0), pz = R(0);
-  if (K == SEG_ARRAYS) {
-    const int64_t m = midx(a, i, j, k);
-    const R *F = static_cast<const R *>(a.force);
-    const R *P = static_cast<const R *>(a.force_prev);
-    Fx = F[m];
-    Fy = F[m + a.ms2];
-    px = P[m];
-    py = P[m + a.ms2];
-    if (L::D == 3) {
-      Fz = F[m + 2 * a.ms2];
-      pz = P[m + 2 * a.ms2];
-    }
-  } else if (K == SEG_UNIFORM) {
-    Fx = px = R(a.uf[0]);
-    Fy = py = R(a.uf[1]);
-    Fz = pz = R(a.uf[2]);
-  }
-  T *fob = static_cast<T *>(a.f_out) + base;
-  if (S == ILBM_STORAGE_F64) {
-    double rho, u, v, w;
-    moments64<L>(reinterpret_cast<double *>(f), double(px), double(py), double(pz), rho, u, v, w);
-    if (L::D != 3) w = 0.0;
-    const bool hf = !(Fx == R(0) && Fy == R(0) && Fz == R(0));
-#pragma unroll
-    for (int q = 0; q < L::Q; ++q)
-      Store<S>::store(fob + a.doff[q],
-                      R(collide64_one<L>(q, double(f[q]), feq64<L>(q, rho, u, v, w), a.tau, u, v, w,
-                                         double(Fx), double(Fy), double(Fz), hf)),
-                      sfac<L, S>(a, q));
-  } else {
-    float drho, u, v, w;
-    moments32<L>(reinterpret_cast<float *>(f), float(px), float(py), float(pz), drho, u, v, w);
-    const Col32 c = col32_setup<L>(drho, u, v, w, a.om32, a.omh32, float(Fx), float(Fy), float(Fz));
-#pragma unroll
-    for (int q = 0; q < L::Q; ++q)
-      Store<S>::store(fob + a.doff[q], R(post32<L>(q, float(f[q]), c)), sfac<L, S>(a, q));
-  }
-}
-
-// The first `ghost_slices` z-slices of the grid push the ghost shell's
-// populations (ghost_push); the rest run one cell per thread.
-template <class L, int S>
-__global__ void __launch_bounds__(256, StepOcc<L, S>::value) k_step(const __grid_constant__ StepArgs a) {
-  if ((int)blockIdx.z < a.ghost_slices) {
-    const uint32_t blk = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-    ghost_push<L, S>(a, blk * blockDim.x + threadIdx.x,
-                     (uint32_t)a.ghost_slices * gridDim.x * gridDim.y * blockDim.x);
-    return;
-  }
-  const int i0 = a.rlo[0] + blockIdx.x * blockDim.x;
-  const int i = i0 + threadIdx.x;
-  const int j = a.rlo[1] + blockIdx.y;
-  const int k = a.rlo[2] + (int)blockIdx.z - a.ghost_slices;
-  const int kind = seg_kind<L>(a, i0, min(i0 + (int)blockDim.x - 1, a.rhi[0]), j, k);
-  if (i > a.rhi[0] || kind == SEG_SKIP) return;
-  if (kind == SEG_ZERO) {
-    cell_fast<L, S, SEG_ZERO>(a, i, j, k);
-  } else if (kind == SEG_UNIFORM) {
-    cell_fast<L, S, SEG_UNIFORM>(a, i, j, k);
-  } else if (kind == SEG_ARRAYS) {
-    cell_fast<L, S, SEG_ARRAYS>(a, i, j, k);
-  } else {
-    if (a.use_skip && in_box(a.slo, a.shi, i, j, k)) return;
-    cell_update<L, S>(a, i, j, k, needs_fixup<L>(a, i, j, k));
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Batched level step: many independent cases (each one box = its level
-// domain, self-filled ghosts) in one persistent launch.  Blocks walk a tile
-// table of row segments and ghost-push chunks over all cases; the arguments
-// of a tile's case are copied to shared memory, so the per-direction offsets
-// stay on chip and cannot alias the population stores.
-// ---------------------------------------------------------------------------
-// the batched step's occupancy target: 5 blocks of 256 (48 registers) for
-// D2Q9 in the 4- and 2-byte forms (measured 5% faster on the 64-case D2Q9
-// batch than 4), as k_step otherwise
-template <class L, int S>
-struct BatchOcc {
-  static constexpr int value = (S != ILBM_STORAGE_F64 && L::Q <= 9) ? 5 : StepOcc<L, S>::value;
-};
-
-template <class L, int S>
-__global__ void __launch_bounds__(256, BatchOcc<L, S>::value)
-    k_step_batch(const StepArgs *__restrict__ args, const StepTile *__restrict__ tiles, int ntiles,
-                 const int *steps, const int *limit) {
-  __shared__ StepArgs sa;
-  int cur = -1;  // every thread walks the same tiles, so this stays block-uniform
-  // strided over the table (block b takes entries b, b + gridDim.x, ...),
-  // which the batch lays out so that the blocks in flight stream through
-  // neighbouring rows together (a contiguous run of rows per block measured
-  // 2.2x slower: the push stores' split lines no longer meet in L2) while a
-  // block keeps to one case; c = -1 marks a filler entry
-  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const StepTile tl = tiles[t];
-    if (tl.c < 0 || steps[tl.c] >= limit[tl.c]) continue;  // filler, or a case that has taken all its steps
-    if (tl.c != cur) {
-      __syncthreads();  // every thread is done with the previous case's arguments
-      const int *src = reinterpret_cast<const int *>(args + tl.c);
-      int *dst = reinterpret_cast<int *>(&sa);
-      for (int w = threadIdx.x; w < (int)(sizeof(StepArgs) / sizeof(int)); w += blockDim.x)
-        dst[w] = src[w];
-      __syncthreads();
-      cur = tl.c;
-    }
-    if (tl.i0 < 0) {
-      ghost_push<L, S>(sa, (uint32_t)(-1 - tl.i0) * blockDim.x + threadIdx.x,
-                       (uint32_t)tl.j * blockDim.x);
-      continue;
-    }
-    // lean row segments as in k_step (a skip box, which single-level cases
-    // do not have, stays on the general path as before)
-    const int i = tl.i0 + threadIdx.x;
-    const int kind = seg_kind<L>(sa, tl.i0, min(tl.i0 + (int)blockDim.x - 1, sa.hi[0]), tl.j, tl.k);
-    if (i > sa.hi[0]) continue;
-    if (kind == SEG_ZERO)
-      cell_fast<L, S, SEG_ZERO>(sa, i, tl.j, tl.k);
-    else if (kind == SEG_UNIFORM)
-      cell_fast<L, S, SEG_UNIFORM>(sa, i, tl.j, tl.k);
-    else if (kind == SEG_ARRAYS)
-      cell_fast<L, S, SEG_ARRAYS>(sa, i, tl.j, tl.k);
-    else
-      cell_update<L, S>(sa, i, tl.j, tl.k, needs_fixup<L>(sa, i, tl.j, tl.k));
-  }
 }
 
 
@@ -1073,6 +411,12 @@ static int fill_args(const ilbm_ctx *ctx, const ilbm_box &b, const ilbm_level_pa
   a.macro_in = b.macro_in;
   a.force = b.force;
   a.force_prev = b.force_prev;
+  const float scale16 = (p && p->f16_scale > 0) ? float(p->f16_scale) : 1024.0f;
+  for (int q = 0; q < ctx->q; ++q) {
+    const bool half = ctx->storage == ILBM_STORAGE_F16_SCALED;
+    a.sf[q] = half ? float(ctx->w[q]) / scale16 : 1.0f;
+    a.si[q] = half ? float(double(scale16) / ctx->w[q]) : 1.0f;
+  }
   if (p) {
     for (int d = 0; d < 3; ++d) {
       a.dlo[d] = (d < D) ? p->domain_lo[d] : 0;
@@ -1094,15 +438,16 @@ static int fill_args(const ilbm_ctx *ctx, const ilbm_box &b, const ilbm_level_pa
     a.self_fill = (p->ghost_mode == ILBM_GHOST_SELF);
     a.use_uniform = p->use_uniform_force;
     for (int d = 0; d < 3; ++d) a.uf[d] = p->uniform_force[d];
-    a.f16_scale = (p->f16_scale > 0) ? float(p->f16_scale) : 1024.0f;
-    // faces that send outgoing populations back into the box: domain faces
-    // that are periodic with self-filled ghosts (wrapped push) or user_1
-    // (halfway bounce-back); every other face leaves them to ghost_push
+    a.f16_scale = scale16;
+    // what each face does with the populations that leave through it
     for (int d = 0; d < D; ++d) {
-      const bool plo = a.periodic[d] ? a.self_fill : (a.bclo[d] == ILBM_BC_USER_1);
-      const bool phi = a.periodic[d] ? a.self_fill : (a.bchi[d] == ILBM_BC_USER_1);
-      a.act_lo[d] = (a.lo[d] == a.dlo[d]) && plo;
-      a.act_hi[d] = (a.hi[d] == a.dhi[d]) && phi;
+      auto face = [&](bool domain_face, int bc) -> int {
+        if (!domain_face) return FACE_BOX;
+        if (a.periodic[d]) return a.self_fill ? FACE_WRAP : FACE_PERIODIC;
+        return bc == ILBM_BC_USER_1 ? FACE_REFLECT : FACE_PHYS;
+      };
+      a.face_lo[d] = face(a.lo[d] == a.dlo[d], a.bclo[d]);
+      a.face_hi[d] = face(a.hi[d] == a.dhi[d], a.bchi[d]);
     }
     int rc = ghost_offsets(D, a);
     if (rc) return rc;
@@ -1116,31 +461,41 @@ static int fill_args(const ilbm_ctx *ctx, const ilbm_box &b, const ilbm_level_pa
         for (int c = 0; c < 6; ++c) a.lb[n][c] = p->level_boxes[6 * n + c];
     }
   } else {
-    a.f16_scale = 1024.0f;
+    a.f16_scale = scale16;
   }
   return ILBM_OK;
 }
 
-// k_step over [rlo, rhi] (minus the skip box), with the ghost shell push in
-// leading z-slices when with_ghosts is set
-template <class L, int S>
-static void launch_cells(ilbm_ctx *ctx, const StepArgs &a_in, cudaStream_t st, bool with_ghosts) {
-  StepArgs a = a_in;
-  const int nx = a.rhi[0] - a.rlo[0] + 1, ny = a.rhi[1] - a.rlo[1] + 1;
-  const int nz = (L::D == 3) ? a.rhi[2] - a.rlo[2] + 1 : 1;
-  if (nx <= 0 || ny <= 0 || nz <= 0) return;
-  const int bx = nx >= 256 ? 256 : ((nx + 31) / 32) * 32;
-  const int gx = (nx + bx - 1) / bx;
-  a.ghost_slices = 0;
-  if (with_ghosts) {
-    // about one ghost cell per thread
-    const int64_t per_slice = (int64_t)gx * ny * bx;
-    const int64_t w = a.goff[3];
-    if (w > 0) a.ghost_slices = (int)std::min<int64_t>(64, (w + per_slice - 1) / per_slice);
-  }
-  dim3 grid(gx, ny, nz + a.ghost_slices);
-  k_step<L, S><<<grid, bx, 0, st>>>(a);
-  ctx->launches++;
+// magic of a division by d (1 <= d < 2^31) of numbers below 2^31 (fast_div):
+// n / d = (floor(n m / 2^32) + n) >> l with l = ceil(log2 d) and
+// m = floor(2^32 (2^l - d) / d) + 1
+DivMagic div_magic(uint32_t d) {
+  uint32_t l = 0;
+  while ((1ull << l) < d) ++l;
+  DivMagic m;
+  m.mul = (uint32_t)(((1ull << 32) * ((1ull << l) - d)) / d + 1);
+  m.shift = l;
+  return m;
+}
+
+// the cells [rlo, rhi] of a launch as a sequence of V-cell vectors; false: empty
+bool plan_vectors(StepArgs &a, int dim, int V) {
+  const int ny = a.rhi[1] - a.rlo[1] + 1, nz = (dim == 3) ? a.rhi[2] - a.rlo[2] + 1 : 1;
+  a.nvec = 0;
+  if (a.rhi[0] < a.rlo[0] || ny <= 0 || nz <= 0) return false;
+  // the vector form goes by the columns that populations land on: those of
+  // the cells and their neighbours inside the box
+  const int x0 = V > 1 ? std::max(a.rlo[0] - 1, a.lo[0]) : a.rlo[0];
+  const int x1 = V > 1 ? std::min(a.rhi[0] + 1, a.hi[0]) : a.rhi[0];
+  a.vx0 = a.lo[0] + (x0 - a.lo[0]) / V * V;
+  a.vpr = (uint32_t)((x1 - a.vx0) / V + 1);
+  a.vny = (uint32_t)ny;
+  a.dvpr = div_magic(a.vpr);
+  a.dvny = div_magic(a.vny);
+  a.nvec = (uint32_t)((int64_t)a.vpr * ny * nz);
+  a.forced = a.force == nullptr && a.force_prev == nullptr && a.use_uniform &&
+             (a.uf[0] != 0.0 || a.uf[1] != 0.0 || a.uf[2] != 0.0);
+  return true;
 }
 
 template <class L, int S>
@@ -1327,7 +682,7 @@ int batch_case_args(const ilbm_ctx *ctx, const ilbm_box &b, const ilbm_level_par
   bb.macro_in = nullptr;
   bb.macro_out = nullptr;
   if ((rc = fill_args(ctx, bb, p, *out))) return rc;
-  out->ghost_slices = 0;
+  out->ghost_blocks = 0;
   return ILBM_OK;
 }
 
@@ -1337,20 +692,38 @@ int batch_ghost_chunks(const ilbm_ctx *, const StepArgs &a, int w) {
 }
 
 template <class L, int S>
-static int launch_step_batch(ilbm_ctx *ctx, const StepArgs *d_args, const StepTile *d_tiles,
-                             int ntiles, int w, int blocks, const int *steps, const int *limit,
-                             cudaStream_t st) {
-  k_step_batch<L, S><<<blocks, w, 0, st>>>(d_args, d_tiles, ntiles, steps, limit);
-  ctx->launches++;
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_fail(e, "batched level step launch");
+static int vec_width_of(const ilbm_ctx *, const StepArgs &a, int *V) {
+  *V = vec_width<L, S>(a);
+  return ILBM_OK;
+}
+
+uint32_t batch_per_block(int V, int w) { return step_vectors_per_block(V, (uint32_t)w); }
+
+// the vector sequences of the cases' cells, V cells per vector for all of them
+int batch_plan(const ilbm_ctx *ctx, StepArgs *args, int n, int *V) {
+  *V = 0;
+  for (int c = 0; c < n; ++c) {
+    int v = 1, rc = ILBM_DISPATCH(ctx, vec_width_of, ctx, args[c], &v);
+    if (rc) return rc;
+    *V = (*V == 0) ? v : std::min(*V, v);
+  }
+  for (int c = 0; c < n; ++c) {
+    const StepArgs &a = args[c];
+    int64_t cells = 1;
+    for (int d = 0; d < ctx->dim; ++d) cells *= a.rhi[d] - a.rlo[d] + 1;
+    if (cells > (1 << 30)) {
+      set_error("batched case: 2^30 cells at most");
+      return ILBM_ERR_RANGE;
+    }
+    plan_vectors(args[c], ctx->dim, *V);
+  }
   return ILBM_OK;
 }
 
 int batch_step_launch(ilbm_ctx *ctx, const StepArgs *d_args, const StepTile *d_tiles, int ntiles,
-                      int w, int blocks, const int *steps, const int *limit, cudaStream_t st) {
+                      int V, int w, int blocks, const int *steps, const int *limit, cudaStream_t st) {
   if (ntiles <= 0) return ILBM_OK;
-  return ILBM_DISPATCH(ctx, launch_step_batch, ctx, d_args, d_tiles, ntiles, w, blocks, steps, limit,
+  return ILBM_DISPATCH(ctx, launch_step_batch, ctx, d_args, d_tiles, ntiles, V, w, blocks, steps, limit,
                        st);
 }
 
@@ -1374,16 +747,9 @@ int batch_band_macro_launch(ilbm_ctx *ctx, const StepArgs *d_args, const BandDes
                        limit, st);
 }
 
-template <class L, int S>
-static int occupancy_step_batch(const ilbm_ctx *, int w, int *per_sm) {
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k_step_batch<L, S>, w, 0);
-  if (e != cudaSuccess) return cuda_fail(e, "batched level step occupancy");
-  return ILBM_OK;
-}
-
 // resident blocks of w threads per SM for the batched level step
-int batch_step_occupancy(const ilbm_ctx *ctx, int w, int *per_sm) {
-  return ILBM_DISPATCH(ctx, occupancy_step_batch, ctx, w, per_sm);
+int batch_step_occupancy(const ilbm_ctx *ctx, int V, int w, int *per_sm) {
+  return ILBM_DISPATCH(ctx, occupancy_step_batch, ctx, V, w, per_sm);
 }
 
 // ---- derived fields and refinement tags ------------------------------------

@@ -10,6 +10,21 @@ namespace ilbm {
 
 constexpr int kMaxLevelBoxes = 64;
 
+// What becomes of populations that leave the box through a face
+// (StepArgs::face_lo / face_hi): 0 is kept for "inside"
+enum FaceState {
+  FACE_WRAP = 1,       // periodic, self-filled: into the image cell
+  FACE_REFLECT = 2,    // user_1: halfway bounce-back
+  FACE_PHYS = 4,       // another physical face: ghost_push delivers what enters
+  FACE_BOX = 8,        // another box of the level (or a coarse-fine face): as above
+  FACE_PERIODIC = 16,  // periodic, caller-filled: as above
+};
+
+// division by a constant through a multiplication (fast_div)
+struct DivMagic {
+  uint32_t mul, shift;
+};
+
 struct StepArgs {
   // box valid region and allocated lower corners
   int lo[3], hi[3];
@@ -40,11 +55,22 @@ struct StepArgs {
   int rlo[3], rhi[3];
   int slo[3], shi[3];
   int use_skip;
-  int ghost_slices;          // leading z-slices of the k_step grid that run ghost_push
+  // the cells of this launch as a sequence of V-cell vectors: first column,
+  // vectors per row, rows per k, vectors in all
+  int vx0;
+  uint32_t vpr, vny, nvec;
+  DivMagic dvpr, dvny;
+  int forced;  // a uniform force on every cell (no force arrays)
+  // F16: per-direction storage factor w_q / scale and its inverse
+  float sf[27], si[27];
+  // blocks of the k_step grid that run ghost_push: one in ghost_every of the
+  // leading ones, ghost_blocks in all
+  uint32_t ghost_blocks, ghost_every;
+  DivMagic dghost;
   // the ghost shell in one sequence: first index of each dimension's slab,
   // and the total (ghost_push)
   uint32_t goff[4];
-  int act_lo[3], act_hi[3];  // face returns outgoing populations (wrap / reflect)
+  int face_lo[3], face_hi[3];  // what a face does with the populations that leave through it (FaceState)
   int nlb;
   int lb[kMaxLevelBoxes][6];
   // with use_mbox, macro_in holds stored values only on [mblo, mbhi]; cells
@@ -61,11 +87,12 @@ __device__ __forceinline__ bool stored_macro_at(const StepArgs &a, int i, int j,
          k <= a.mbhi[2];
 }
 
-// One work item of the batched level step (k_step_batch): a row segment of
-// blockDim.x cells of case c starting at (i0, j, k), or, when i0 < 0, chunk
-// (-1 - i0) of the case's ghost shell push, which has j chunks in all.
+// One work item of the batched level step (k_step_batch): blockDim.x vectors
+// of case c from vector `first` on, or, with ghosts > 0, the ghost shell cells
+// from `first` on in strides of `ghosts`; c = -1: a filler.
 struct StepTile {
-  int c, i0, j, k;
+  int c;
+  uint32_t first, ghosts;
 };
 
 // Support band of an immersed body on a case's level (EV: 3 velocity

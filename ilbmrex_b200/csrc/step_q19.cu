@@ -1,0 +1,5 @@
+// Level-step kernels, D3Q19 in the 4- and 2-byte storage forms.
+#include "level_step.cuh"
+
+ILBM_STEP_INSTANCE(19, ILBM_STORAGE_F32_SHIFT)
+ILBM_STEP_INSTANCE(19, ILBM_STORAGE_F16_SCALED)

@@ -1,0 +1,5 @@
+// Level-step kernels, D2Q9 in the 4- and 2-byte storage forms.
+#include "level_step.cuh"
+
+ILBM_STEP_INSTANCE(9, ILBM_STORAGE_F32_SHIFT)
+ILBM_STEP_INSTANCE(9, ILBM_STORAGE_F16_SCALED)
