@@ -71,6 +71,7 @@ struct AdvanceSplit {
   ilbm_level_params q;  // the level's parameters with the body's force region
   int lo[3], hi[3];     // the body's band
   bool serial;          // no overlap: forcing first, then the whole step
+  bool tail;            // work of the side stream after the exported force (ev_done)
 };
 int advance_begin(ilbm_ctx *ctx, const ilbm_box *box, const ilbm_level_params *p, ilbm_ib *ib,
                   double dt, double time, AdvanceSplit *sp);

@@ -28,6 +28,7 @@
 #include "batch_internal.h"
 #include "ilbm_common.cuh"
 #include "state_internal.h"
+#include "step_device.cuh"
 
 namespace cgrp = cooperative_groups;
 
@@ -46,6 +47,10 @@ int level_step_split(ilbm_ctx *ctx, const ilbm_box &b, const ilbm_level_params *
 }
 
 using namespace ilbm;
+
+// (ib_chain.cuh) bodies whose forcing chain is one launch
+static constexpr int kChainMaxMarkers = 512, kChainMaxCg = 448;
+static constexpr int64_t kChainMaxBand = 65536;
 
 namespace {
 
@@ -2279,6 +2284,7 @@ int ilbm_ib_create(ilbm_ctx *ctx, const ilbm_ib_params *p, const ilbm_level_geom
   // band fields finite everywhere (a fixed body forms them on its stencils only)
   cudaMemsetAsync(ib->d_EV, 0, 3 * (size_t)ib->nb * sizeof(double), ctx->stream);
   cudaMemsetAsync(ib->d_RHO, 0, (size_t)ib->nb * sizeof(double), ctx->stream);
+  cudaMemsetAsync(ib->d_EFI, 0, 3 * (size_t)ib->nb * sizeof(double), ctx->stream);
   if ((rc = dmalloc(ib, &ib->d_recscr, force_record_scratch()))) {
     ilbm_ib_destroy(ib);
     return rc;
@@ -2456,6 +2462,10 @@ static int ib_box_table(ilbm_ib *ib, const ilbm_box *boxes, int nbox, const ilbm
   return ILBM_OK;
 }
 
+// the chain of a small body on one box in one launch (ib_chain.cuh)
+static int launch_chain(ilbm_ib *ib, const ilbm_box &box, const ilbm_level_params *lp, const IBArgs &a,
+                        int mode, cudaStream_t s);
+
 static int ib_update(ilbm_ib *ib, const ilbm_box *boxes, int nbox, const ilbm_level_params *lp,
                      double dt, double time, cudaStream_t s, bool defer_sum) {
   if (!ib || !boxes || nbox < 1 || !lp) {
@@ -2498,6 +2508,21 @@ static int ib_update(ilbm_ib *ib, const ilbm_box *boxes, int nbox, const ilbm_le
   bool periodic_band = false;
   for (int d = 0; d < ib->dim; ++d)
     periodic_band = periodic_band || (ib->g.periodic[d] && ib->blo[d] < 0);
+  const bool use_dense_ = ivc_ && ib->dense && !ib->moving && ib->p.ivc_rebuild_matrix == 0 &&
+                          ib->ivc_solver != ILBM_IVC_CG;
+  // A small body takes its whole chain in one launch: a stored inverse once it
+  // is built (the first step, below, builds it), a CG solve where the operator
+  // is rebuilt every step anyway, or explicit coupling.  Larger bodies keep a
+  // launch per stage over the whole device.
+  if (!multi && single_ && ib->nb <= kChainMaxBand &&
+      ib->n <= (ivc_ && !use_dense_ ? kChainMaxCg : kChainMaxMarkers) &&
+      (!ivc_ || (use_dense_ ? ib->dense_ready : (ib->moving || ib->p.ivc_rebuild_matrix > 0)))) {
+    int rc = launch_chain(ib, *box, lp, make_args(ib, dt, time), !ivc_ ? 0 : (use_dense_ ? 1 : 2), s);
+    if (rc) return rc;
+    ib->csr_ready = ib->csr_ready || (ivc_ && !use_dense_);  // (a batch rebuilds such an operator itself)
+    ib->fsum_deferred = false;
+    return ILBM_OK;
+  }
   // EulerVel / rho on the band (:1541-1566, FillBoundary :702-703).  A body
   // whose markers do not move reads them only on the cells its stencils
   // reach (its spreading table): only those are formed.  The rest of the band
@@ -2689,6 +2714,7 @@ int advance_begin(ilbm_ctx *ctx, const ilbm_box *box, const ilbm_level_params *p
   bool band_inside = p->nlevel_boxes <= 1 && box->f_in != box->f_out;
   for (int d = 0; d < ctx->dim; ++d)
     band_inside = band_inside && sp->lo[d] >= box->lo[d] && sp->hi[d] <= box->hi[d];
+  sp->tail = false;
   sp->serial = (p->ghost_mode != ILBM_GHOST_SELF && !band_inside);
   if (sp->serial) return ib_update(ib, box, 1, &sp->q, dt, time, ctx->stream, false);
   // validate like ilbm_level_step does before anything is launched
@@ -2706,6 +2732,8 @@ int advance_begin(ilbm_ctx *ctx, const ilbm_box *box, const ilbm_level_params *p
   e = cudaEventRecord(ctx->ev_join, ctx->side);
   if (e != cudaSuccess) return cuda_fail(e, "ilbm_advance_level join");
   // the marker force sum runs beside the band's collide-stream
+  sp->tail = ib->fsum_deferred;
+  if (!sp->tail) return ILBM_OK;
   if ((rc = ib_finish(ib, ctx->side))) return rc;
   e = cudaEventRecord(ctx->ev_done, ctx->side);
   if (e != cudaSuccess) return cuda_fail(e, "ilbm_advance_level done");
@@ -2717,7 +2745,7 @@ int advance_end(ilbm_ctx *ctx, const ilbm_box *box, const AdvanceSplit *sp) {
   // the collide-stream of every cell outside the band, then the band once
   // the body's forcing is in
   int rc = level_step_split(ctx, *box, &sp->q, sp->lo, sp->hi, ctx->ev_join);
-  if (rc) return rc;
+  if (rc || !sp->tail) return rc;
   cudaError_t e = cudaStreamWaitEvent(ctx->stream, ctx->ev_done, 0);
   if (e != cudaSuccess) return cuda_fail(e, "ilbm_advance_level wait");
   return ILBM_OK;
@@ -2939,7 +2967,15 @@ struct IBCase {
   double *tw;         // the step's marker weight table (kTabStride per marker) and cells
   int4 *tc;
   int tile0, ntile;   // the case's band tiles in the batch's tile list
+  // markers that do not move: their weights, and the band cells their
+  // stencils reach with the markers' entries (the fixed-order spreading)
+  const SpreadW *sw;
+  const int64_t *gcell;
+  const int *growptr, *gent;
+  int gcells;
 };
+
+#include "ib_chain.cuh"
 
 // a case that has taken all the steps it was added for sits out
 __device__ __forceinline__ bool live(const int *steps, const int *limit, int c) {
@@ -3124,6 +3160,72 @@ __global__ void __launch_bounds__(kRecThreads) k_b_record(const IBCase *cs, int 
 }
 
 }  // namespace
+
+// what the chain needs of a body
+static void chain_case(ilbm_ib *ib, const IBArgs &a, int mode, IBCase &k) {
+  std::memset(&k, 0, sizeof(k));
+  k.a = a;
+  k.xyz = ib->d_xyz;
+  k.ref = ib->d_ref;
+  k.tgt = ib->d_tgt;
+  k.uvw = ib->d_uvw;
+  k.F = ib->d_F;
+  k.EFI = ib->d_EFI;
+  k.fsum = ib->d_fsum;
+  k.status = ib->d_status;
+  k.iters = ib->d_iters;
+  k.mode = mode;
+  k.moving = ib->moving ? 1 : 0;
+  for (int d = 0; d < ib->dim; ++d)
+    k.periodic_band = k.periodic_band || (ib->g.periodic[d] && ib->blo[d] < 0);
+  k.X = ib->d_X;
+  k.Xh = ib->d_Xh;
+  k.hist = ib->d_hist;
+  k.reg = ib->p.ivc_diag_reg;
+  k.cg_tol = ivc_cg_tolerance(ib->ctx->storage);
+  k.Ainv = ib->d_Ainv;
+  k.Ainv32 = ib->d_Ainv32;
+  k.rhs = ib->d_rhs;
+  k.ld = ib->ld;
+  k.tw = ib->d_tw;
+  k.tc = ib->d_tc;
+  if (ib->gather && ib->sw_ready) {
+    k.sw = static_cast<const SpreadW *>(ib->d_sw);
+    k.gcell = ib->d_gcell;
+    k.growptr = ib->d_growptr;
+    k.gent = ib->d_gent;
+    k.gcells = ib->gather_cells;
+  }
+}
+
+template <class L, int S>
+static int launch_chain_of(ilbm_ctx *ctx, const ChainArgs &c, cudaStream_t s) {
+  cudaError_t e = cudaFuncSetAttribute(k_ib_chain<L, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)chain_shared(2, kChainMaxCg));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_ib_chain<L, S>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e != cudaSuccess) return cuda_fail(e, "body forcing: shared memory");
+  k_ib_chain<L, S><<<kChainCtas, kChainThreads, chain_shared(c.k.mode, c.k.a.n), s>>>(c);
+  ctx->launches++;
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_fail(e, "body forcing");
+  return ILBM_OK;
+}
+
+static int launch_chain(ilbm_ib *ib, const ilbm_box &box, const ilbm_level_params *lp, const IBArgs &a,
+                        int mode, cudaStream_t s) {
+  ilbm_ctx *ctx = ib->ctx;
+  ChainArgs c;
+  int rc = box_step_args(ctx, box, lp, &c.s);
+  if (rc) return rc;
+  if (ib->gather && !ib->sw_ready) {
+    k_spread_weights<<<(ib->n + 127) / 128, 128, 0, s>>>(a, ib->d_xyz, static_cast<SpreadW *>(ib->d_sw));
+    ctx->launches++;
+    ib->sw_ready = true;
+  }
+  chain_case(ib, a, mode, c.k);
+  return ILBM_DISPATCH(ctx, launch_chain_of, ctx, c, s);
+}
 
 namespace ilbm {
 

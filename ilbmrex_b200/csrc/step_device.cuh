@@ -1,6 +1,7 @@
 // Device helpers of the level step shared by its kernels (level_step.cuh) and
 // the macro, initialisation and band kernels (lbm_step.cu): cell indices,
-// population and force loads, the ghost rules of a self-filled level.
+// population and force loads, the ghost rules of a self-filled level, rho and u
+// of a cell of the immersed boundary's band.
 #pragma once
 
 #include "ilbm_common.cuh"
@@ -139,6 +140,94 @@ __device__ __forceinline__ int ghost_rule(const StepArgs &a, const int *g, int *
   src[1] = min(max(g[1], a.dlo[1]), a.dhi[1]);
   src[2] = (L::D == 3) ? min(max(g[2], a.dlo[2]), a.dhi[2]) : 0;
   return 0;
+}
+
+// ---------------------------------------------------------------------------
+// Band macro for the immersed boundary: rho, u, v, w (FP64) on the cells of
+// the IB support band, including up to two ghost layers outside the domain.
+// Valid cells: from macro_in, or from f^n and F^{n-1} (the value the
+// reference's macro pass stored).  Ghost cells: FillPatchMacro semantics
+// (periodic image, foextrap, macroBcFill: user_2 mirrored state, user_1 /
+// ext_dir prescribed state; Source/BC/bc_fill.H:69-142, 263-301).
+// ---------------------------------------------------------------------------
+template <class L, int S>
+__device__ void macro_at(const StepArgs &a, int i, int j, int k, double *m4) {
+  if (stored_macro_at(a, i, j, k)) {
+    const int64_t m = midx(a, i, j, k);
+    if (S == ILBM_STORAGE_F64) {
+      m4[0] = ldm<double>(a.macro_in, m);
+      m4[1] = ldm<double>(a.macro_in, m + a.ms2);
+      m4[2] = ldm<double>(a.macro_in, m + 2 * a.ms2);
+      m4[3] = (L::D == 3) ? ldm<double>(a.macro_in, m + 3 * a.ms2) : 0.0;
+    } else {
+      m4[0] = ldm<float>(a.macro_in, m);
+      m4[1] = ldm<float>(a.macro_in, m + a.ms2);
+      m4[2] = ldm<float>(a.macro_in, m + 2 * a.ms2);
+      m4[3] = (L::D == 3) ? ldm<float>(a.macro_in, m + 3 * a.ms2) : 0.0;
+    }
+    return;
+  }
+  const int64_t b = fidx(a, i, j, k);
+  if (S == ILBM_STORAGE_F64) {
+    double f[L::Q];
+#pragma unroll
+    for (int q = 0; q < L::Q; ++q) f[q] = ldf<L, S>(a, b, q);
+    double px, py, pz;
+    load_force<L, double>(a, a.force_prev, i, j, k, px, py, pz);
+    moments64<L>(f, px, py, pz, m4[0], m4[1], m4[2], m4[3]);
+    if (L::D != 3) m4[3] = 0.0;
+  } else {
+    float g[L::Q];
+#pragma unroll
+    for (int q = 0; q < L::Q; ++q) g[q] = ldf<L, S>(a, b, q);
+    float px, py, pz, drho, u, v, w;
+    load_force<L, float>(a, a.force_prev, i, j, k, px, py, pz);
+    moments32<L>(g, px, py, pz, drho, u, v, w);
+    m4[0] = 1.0 + double(drho);
+    m4[1] = u;
+    m4[2] = v;
+    m4[3] = (L::D == 3) ? double(w) : 0.0;
+  }
+}
+
+// rho, u, v, w of one band cell
+template <class L, int S>
+__device__ __forceinline__ void band_macro_value(const StepArgs &a, int i, int j, int k, double *m4) {
+  const int g[3] = {i, j, k};
+  const bool in = in_domain<L>(a, g[0], g[1], g[2]);
+  if (in || (a.macro_in && !a.self_fill)) {
+    // caller-filled macros carry their own ghost values
+    macro_at<L, S>(a, g[0], g[1], L::D == 3 ? g[2] : 0, m4);
+    return;
+  }
+  int src[3], bd = 0, lo_side = 1;
+  const int kind = ghost_rule<L>(a, g, src, bd, lo_side);
+  macro_at<L, S>(a, src[0], src[1], L::D == 3 ? src[2] : 0, m4);
+  const double *bv = lo_side ? a.bvlo[bd] : a.bvhi[bd];
+  if (kind == 3) {
+    m4[0] = fmax(1.0e-20, X::sub(X::mul(2.0, bv[0]), m4[0]));
+    m4[1] = X::sub(X::mul(2.0, bv[1]), m4[1]);
+    m4[2] = X::sub(X::mul(2.0, bv[2]), m4[2]);
+    m4[3] = X::sub(X::mul(2.0, bv[3]), m4[3]);
+  } else if (kind == 1 || kind == 2) {
+    m4[0] = bv[0];
+    m4[1] = bv[1];
+    m4[2] = bv[2];
+    m4[3] = bv[3];
+  }
+}
+
+template <class L, int S>
+__device__ __forceinline__ void band_macro_cell(const StepArgs &a, int blo0, int blo1, int blo2,
+                                                int bn0, int bn1, int64_t nb, int64_t t,
+                                                double *EV, double *RHO) {
+  double m4[4];
+  band_macro_value<L, S>(a, blo0 + (int)(t % bn0), blo1 + (int)((t / bn0) % bn1),
+                         blo2 + (int)(t / ((int64_t)bn0 * bn1)), m4);
+  EV[t] = m4[1];
+  EV[t + nb] = m4[2];
+  EV[t + 2 * nb] = (L::D == 3) ? m4[3] : 0.0;
+  RHO[t] = m4[0];
 }
 
 }  // namespace ilbm
