@@ -1315,84 +1315,78 @@ __global__ void __launch_bounds__(128) k_interp(IBArgs a, const double *xyz, con
 // velocity_interpolation_cic sums a marker's stencil sequentially (i, then
 // j, then k innermost, IBMarkerDF.cpp:612-695); force_spreading adds the
 // markers' contributions to each cell in marker order (the loop over
-// particles, :1331-1448).  The kernels below keep both orders: one thread per
+// particles, :1331-1448).  The kernels below keep both orders: a warp per
 // marker for the interpolation, and for a body whose markers do not move a
 // gather over a cell -> marker table built once (markers in increasing
 // order), so each cell's force is the reference's sum, computed once, with
 // no atomics.  FP64 results then equal the reference's bit for bit wherever
 // the rest of the chain does (explicit and explicit_diag coupling).
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void interp_seq(const IBArgs &a, int m, const double *xyz,
+// A warp per marker: lane l forms the terms of points l, l + 32, ... (all
+// loads of a round in flight together), then every lane adds them in point
+// order, which is the reference's loop order.  (One thread per marker walked
+// the 125 points with a load each and evaluated the fifteen kernel values one
+// after another: 50 us for the 804 markers of the 128 x 64 x 64 sphere against
+// 13 us; 16.7 -> 11.3 us for the gather below
+// with four entries' loads in flight.)
+__device__ __forceinline__ void interp_seq(const IBArgs &a, int m, int lane, const double *xyz,
                                            const double *EV, double *uvw, int *status,
                                            const double *tgt, double *rhs, int ld) {
   const double px = xyz[m], py = xyz[m + a.n], pz = xyz[m + 2 * a.n];
   const double d = (a.dim == 3) ? X::mul(X::mul(a.dx[0], a.dx[1]), a.dx[2]) : X::mul(a.dx[0], a.dx[1]);
-  const int i0 = cell_of(px, a.plo[0], a.dx[0]), j0 = cell_of(py, a.plo[1], a.dx[1]);
-  const int k0 = (a.dim == 3) ? cell_of(pz, a.plo[2], a.dx[2]) : 0;
-  double wx[5], wy[5], wz[5];
-#pragma unroll
-  for (int o = 0; o < 5; ++o) {
-    wx[o] = delta_fn(cell_center(a.plo[0], i0 + o - 2, a.dx[0]), px, a.dx[0], a.kt);
-    wy[o] = delta_fn(cell_center(a.plo[1], j0 + o - 2, a.dx[1]), py, a.dx[1], a.kt);
-    wz[o] = (a.dim == 3) ? delta_fn(cell_center(a.plo[2], k0 + o - 2, a.dx[2]), pz, a.dx[2], a.kt) : 1.0;
-  }
+  int i0, j0, k0;
+  double wx, wy, wz;
+  marker_weights(a, px, py, pz, lane, i0, j0, k0, wx, wy, wz);
   const int ilo = a.dlo[0] - 2, ihi = a.dhi[0] + 2, jlo = a.dlo[1] - 2, jhi = a.dhi[1] + 2;
   const int klo = (a.dim == 3) ? a.dlo[2] - 2 : 0, khi = (a.dim == 3) ? a.dhi[2] + 2 : 0;
-  const int nk = (a.dim == 3) ? 5 : 1;
-  double u = 0.0, v = 0.0, w = 0.0, part = 0.0;
-  bool outside = false;
-  for (int ii = 0; ii < 5; ++ii) {
-    const int ip = i0 + ii - 2;
-    if (ip < ilo || ip > ihi || wx[ii] == 0.0) continue;
-    for (int jj = 0; jj < 5; ++jj) {
-      const int jp = j0 + jj - 2;
-      if (jp < jlo || jp > jhi || wy[jj] == 0.0) continue;
-      for (int kk = 0; kk < nk; ++kk) {
-        const int kp = (a.dim == 3) ? k0 + kk - 2 : 0;
-        if (kp < klo || kp > khi) continue;
-        const double dvl = (a.dim == 3) ? X::mul(X::mul(wx[ii], wy[jj]), wz[kk]) : X::mul(wx[ii], wy[jj]);
-        // points outside the kernel's support add signed zeros to sums that
-        // start at +0: skipping them leaves every sum bit for bit as it was
-        if (dvl == 0.0) continue;
-        if (!in_band(a, ip, jp, kp)) {
-          outside = true;
-          continue;
-        }
+  const int npts = (a.dim == 3) ? 125 : 25;
+  double s[4] = {0.0, 0.0, 0.0, 0.0};  // u, v, w, partition
+  for (int t0 = 0; t0 < npts; t0 += 32) {
+    const int t = t0 + lane, tt = t < npts ? t : 0;
+    const int ii = tt / ((a.dim == 3) ? 25 : 5), jj = (tt / ((a.dim == 3) ? 5 : 1)) % 5;
+    const int kk = (a.dim == 3) ? tt % 5 : 2;
+    const double tU = __shfl_sync(0xffffffffu, wx, ii), tV = __shfl_sync(0xffffffffu, wy, jj);
+    const double tW = __shfl_sync(0xffffffffu, wz, kk);
+    const int ip = i0 + ii - 2, jp = j0 + jj - 2, kp = (a.dim == 3) ? k0 + kk - 2 : 0;
+    const double dvl = (a.dim == 3) ? X::mul(X::mul(tU, tV), tW) : X::mul(tU, tV);
+    // points outside the kernel's support or the clip box add zeros to sums
+    // that start at +0: every sum stays bit for bit the reference's
+    double c[4] = {0.0, 0.0, 0.0, 0.0};
+    if (t < npts && dvl != 0.0 && ip >= ilo && ip <= ihi && jp >= jlo && jp <= jhi && kp >= klo && kp <= khi) {
+      if (!in_band(a, ip, jp, kp)) {
+        atomicOr(status, 1);
+      } else {
         const int64_t e = bidx(a, ip, jp, kp);
-        part = X::add(part, X::mul(dvl, d));
-        u = X::add(u, X::mul(X::mul(dvl, EV[e]), d));
-        v = X::add(v, X::mul(X::mul(dvl, EV[e + a.nb]), d));
-        if (a.dim == 3) w = X::add(w, X::mul(X::mul(dvl, EV[e + 2 * a.nb]), d));
+        c[0] = X::mul(X::mul(dvl, EV[e]), d);
+        c[1] = X::mul(X::mul(dvl, EV[e + a.nb]), d);
+        if (a.dim == 3) c[2] = X::mul(X::mul(dvl, EV[e + 2 * a.nb]), d);
+        c[3] = X::mul(dvl, d);
       }
     }
+    const int cnt = min(32, npts - t0);
+    for (int l = 0; l < cnt; ++l)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) s[q] = X::add(s[q], __shfl_sync(0xffffffffu, c[q], l));
   }
-  if (outside) atomicOr(status, 1);
-  if (a.renorm_interp && part > 0.0) {
-    u = X::div(u, part);
-    v = X::div(v, part);
-    w = X::div(w, part);
-  }
-  u = X::add(uvw[m], u);
-  v = X::add(uvw[m + a.n], v);
-  w = X::add(uvw[m + 2 * a.n], w);
-  uvw[m] = u;
-  uvw[m + a.n] = v;
-  uvw[m + 2 * a.n] = w;
-  if (rhs) {
-    double Ux, Uy, Uz;
-    target_of(a, m, xyz, tgt, Ux, Uy, Uz);
-    rhs[m] = X::div(X::sub(Ux, u), a.dt);
-    rhs[m + ld] = X::div(X::sub(Uy, v), a.dt);
-    rhs[m + 2 * ld] = X::div(X::sub(Uz, w), a.dt);
+  if (lane != 0) return;
+  if (a.renorm_interp && s[3] > 0.0)
+    for (int q = 0; q < 3; ++q) s[q] = X::div(s[q], s[3]);
+  double U[3] = {0.0, 0.0, 0.0};
+  if (rhs) target_of(a, m, xyz, tgt, U[0], U[1], U[2]);
+  for (int q = 0; q < 3; ++q) {
+    s[q] = X::add(uvw[m + q * a.n], s[q]);
+    uvw[m + q * a.n] = s[q];
+    if (rhs) rhs[m + q * ld] = X::div(X::sub(U[q], s[q]), a.dt);
   }
 }
 
 __global__ void __launch_bounds__(128) k_interp_seq(IBArgs a, const double *xyz, const double *EV,
                                                     double *uvw, int *status, const double *tgt,
                                                     double *rhs, int ld) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const int m = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (m >= a.n) return;
-  interp_seq(a, m, xyz, EV, uvw, status, tgt, rhs, ld);
+  interp_seq(a, m, lane, xyz, EV, uvw, status, tgt, rhs, ld);
 }
 
 // per marker: its five kernel weights per direction and the spreading scale
@@ -1446,21 +1440,37 @@ __global__ void __launch_bounds__(128) k_spread_weights(IBArgs a, const double *
 // jj << 3 | kk.
 // the force of gather row r: its markers' contributions in increasing order
 __device__ __forceinline__ void gather_row(const IBArgs &a, const SpreadW *__restrict__ W,
-                                           const double *__restrict__ F,
+                                           const double *F,
                                            const int *__restrict__ rowptr,
                                            const int *__restrict__ ent, int r, double &ax,
                                            double &ay, double &az) {
   ax = ay = az = 0.0;
-  for (int e = rowptr[r]; e < rowptr[r + 1]; ++e) {
-    const int pk = ent[e];
-    const int m = pk >> 9, ii = (pk >> 6) & 7, jj = (pk >> 3) & 7, kk = pk & 7;
-    const SpreadW &w = W[m];
-    const double t3 = (a.dim == 3) ? X::mul(X::mul(w.w[0][ii], w.w[1][jj]), w.w[2][kk])
-                                   : X::mul(w.w[0][ii], w.w[1][jj]);
-    const double dvl = X::mul(t3, w.scale);
-    ax = X::add(ax, X::mul(dvl, X::mul(F[m], a.dv)));
-    ay = X::add(ay, X::mul(dvl, X::mul(F[m + a.n], a.dv)));
-    if (a.dim == 3) az = X::add(az, X::mul(dvl, X::mul(F[m + 2 * a.n], a.dv)));
+  const int e1 = rowptr[r + 1];
+  // four entries' loads in flight before their sums, which keep the order
+  for (int e0 = rowptr[r]; e0 < e1; e0 += 4) {
+    double dvl[4], fx[4], fy[4], fz[4];
+    int pk[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) pk[u] = (e0 + u < e1) ? ent[e0 + u] : -1;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (pk[u] < 0) continue;
+      const int m = pk[u] >> 9, ii = (pk[u] >> 6) & 7, jj = (pk[u] >> 3) & 7, kk = pk[u] & 7;
+      const SpreadW &w = W[m];
+      const double t3 = (a.dim == 3) ? X::mul(X::mul(w.w[0][ii], w.w[1][jj]), w.w[2][kk])
+                                     : X::mul(w.w[0][ii], w.w[1][jj]);
+      dvl[u] = X::mul(t3, w.scale);
+      fx[u] = F[m];
+      fy[u] = F[m + a.n];
+      fz[u] = (a.dim == 3) ? F[m + 2 * a.n] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (pk[u] < 0) continue;
+      ax = X::add(ax, X::mul(dvl[u], X::mul(fx[u], a.dv)));
+      ay = X::add(ay, X::mul(dvl[u], X::mul(fy[u], a.dv)));
+      if (a.dim == 3) az = X::add(az, X::mul(dvl[u], X::mul(fz[u], a.dv)));
+    }
   }
 }
 
@@ -2583,7 +2593,7 @@ static int ib_update(ilbm_ib *ib, const ilbm_box *boxes, int nbox, const ilbm_le
     if (!fresh) k_markers<<<nblk, nthr, 0, s>>>(a, ib->d_xyz, ib->d_ref, ib->d_tgt, ib->d_uvw, ib->d_F);
     if (any_periodic_band) k_fill_boundary<<<gb, 256, 0, s>>>(a, ib->d_EV);
     if (ordered)
-      k_interp_seq<<<nblk, nthr, 0, s>>>(a, ib->d_xyz, ib->d_EV, ib->d_uvw, ib->d_status, ib->d_tgt,
+      k_interp_seq<<<wblk, 128, 0, s>>>(a, ib->d_xyz, ib->d_EV, ib->d_uvw, ib->d_status, ib->d_tgt,
                                          use_dense ? ib->d_rhs : nullptr, ib->ld);
     else if (table)
       k_interp_w<<<wblk, 128, 0, s>>>(a, ib->d_xyz, sw, ib->d_EV, ib->d_uvw, ib->d_F, fresh ? 1 : 0,

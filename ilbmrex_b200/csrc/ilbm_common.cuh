@@ -233,6 +233,152 @@ __device__ __forceinline__ void moments64(const double *f, double Fx, double Fy,
   w = X::div(X::add(m3, X::mul(0.5, Fz)), r);
 }
 
+// ---------------------------------------------------------------------------
+// The FP64 collision of a cell, bit for bit the functions above with fewer
+// operations: products with a lattice component are signs or vanish, a
+// direction and its opposite share their even terms, and the quotients, all
+// by numbers that are the same for every cell (tau, cs2, cs2^2), come from the
+// divisor's correctly rounded reciprocal y by Markstein's scheme (P. Markstein,
+// IBM J. Res. Dev. 34, 1990; Muller et al., Handbook of Floating-Point
+// Arithmetic): q0 = a y, q1 = q0 + (a - b q0) y is faithful, and
+// q1 + (a - b q1) y is the correctly rounded a / b, each step one fused
+// multiply-add, as long as nothing overflows or goes subnormal.  Cells where
+// something might (or where rho or u is not an ordinary number) report it and
+// are redone with the functions above.  About 350 FP64 instructions per D3Q19
+// cell instead of about 650, which FP64 steps are bound by beside the memory
+// traffic: the D3Q19 step of the 128 x 64 x 64 sphere 50 -> 37 us (24.7 us of
+// traffic), its body's band with forces 25 -> 7 us.
+// ---------------------------------------------------------------------------
+struct Tau64 {
+  double tau, inv;  // tau and 1 / tau rounded to nearest
+  double fac;       // 1 - 0.5 / tau, rounded as collide64v does
+};
+
+// outside 2^-959 .. 2^960, not counting zero
+__device__ __forceinline__ bool unordinary(double a) {
+  const unsigned hi = (unsigned)__double2hiint(a) & 0x7fffffffu, lo = (unsigned)__double2loint(a);
+  return hi - (64u << 20) > (1919u << 20) && (hi | lo) != 0u;
+}
+__device__ __forceinline__ double div_by(double a, double b, double y, bool &odd) {
+  odd = odd || unordinary(a);
+  double q = X::mul(a, y);
+  q = __fma_rn(__fma_rn(-b, q, a), y, q);
+  return __fma_rn(__fma_rn(-b, q, a), y, q);
+}
+
+template <class L>
+__host__ __device__ constexpr int pair_sign(int q);
+
+// c'.x of the canonical member of q's pair: the nonzero terms in x, y, z order
+template <class L>
+__device__ __forceinline__ double canon_dot64(int q, double x, double y, double z) {
+  const int s = pair_sign<L>(q), c[3] = {s * L::cx(q), s * L::cy(q), s * L::cz(q)};
+  const double v[3] = {x, y, z};
+  double r = 0.0;
+  bool first = true;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    if (c[d] == 0) continue;
+    r = first ? v[d] : (c[d] > 0 ? X::add(r, v[d]) : X::sub(r, v[d]));  // the first one is +1
+    first = false;
+  }
+  return r;
+}
+
+// moments64 without the products with 0 and +-1
+template <class L>
+__device__ __forceinline__ void moments64_fast(const double *f, double Fx, double Fy, double Fz, double &rho,
+                                               double &u, double &v, double &w) {
+  double r = 0.0, m[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+  for (int q = 0; q < L::Q; ++q) {
+    const int c[3] = {L::cx(q), L::cy(q), L::cz(q)};
+    r = X::add(r, f[q]);
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      if (c[d]) m[d] = c[d] > 0 ? X::add(m[d], f[q]) : X::sub(m[d], f[q]);
+  }
+  rho = r;
+  u = X::div(X::add(m[0], X::mul(0.5, Fx)), r);
+  v = X::div(X::add(m[1], X::mul(0.5, Fy)), r);
+  w = (L::D == 3) ? X::div(X::add(m[2], X::mul(0.5, Fz)), r) : 0.0;
+}
+
+// f -> f* in place from rho, u (FORCED: the Guo increment of F where hf); true
+// if the cell has to be redone (f is then not to be used)
+template <class L, bool FORCED>
+__device__ __forceinline__ bool collide64_cell(double (&f)[L::Q], const Tau64 &t, double rho, double u, double v,
+                                               double w, double Fx, double Fy, double Fz, bool hf) {
+  // tau below 2^50, rho within 2^-500 .. 2^500, |u| below 2^100 (a NaN fails the tests)
+  bool odd = !(t.tau < 0x1p50 && rho > 0x1p-500 && rho < 0x1p500 && fabs(u) < 0x1p100 && fabs(v) < 0x1p100 && fabs(w) < 0x1p100);
+  const double uv = (L::D == 3) ? X::add(X::add(X::mul(u, u), X::mul(v, v)), X::mul(w, w))
+                                : X::add(X::mul(u, u), X::mul(v, v));
+  const double uv15 = X::mul(1.5, uv);
+  constexpr double cs2 = 1.0 / 3.0, c4 = cs2 * cs2, ycs2 = 1.0 / cs2, yc4 = 1.0 / c4;
+  const double F[3] = {Fx, Fy, Fz}, U[3] = {u, v, w};
+  double ax[3][3];  // (c - u) / cs2 for c = -1, 0, 1
+  if (FORCED && hf) {
+#pragma unroll
+    for (int d = 0; d < L::D; ++d)
+#pragma unroll
+      for (int c = -1; c <= 1; ++c) ax[d][c + 1] = div_by(X::sub(double(c), U[d]), cs2, ycs2, odd);
+  }
+#pragma unroll
+  for (int q = 0; q < L::Q; ++q) {
+    const int o = opposite<L>(q);
+    if (o < q) continue;  // done with its pair
+    const double wr = X::mul(L::w(q), rho);
+    const double eu = canon_dot64<L>(q, u, v, w);  // of the canonical member; its negative for the other
+    const double eu3 = X::mul(3.0, eu), eu45 = X::mul(X::mul(4.5, eu), eu);
+    double e4 = 0.0;
+    if (FORCED && hf) e4 = div_by(eu, c4, yc4, odd);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int p = h ? o : q;
+      if (h && o == q) continue;
+      const bool pos = (o == q) || pair_sign<L>(p) > 0;
+      const double a = pos ? X::add(1.0, eu3) : X::sub(1.0, eu3);
+      const double fe = X::mul(wr, X::sub(X::add(a, eu45), uv15));
+      double r = X::sub(f[p], div_by(X::sub(f[p], fe), t.tau, t.inv, odd));
+      if (FORCED && hf) {
+        const int c[3] = {L::cx(p), L::cy(p), L::cz(p)};
+        const double ee = pos ? e4 : -e4;
+        double S = 0.0;
+#pragma unroll
+        for (int d = 0; d < L::D; ++d) {
+          const double term = c[d] == 0 ? ax[d][1] : X::add(ax[d][c[d] + 1], c[d] > 0 ? ee : -ee);
+          S = d == 0 ? X::mul(term, F[d]) : X::add(S, X::mul(term, F[d]));
+        }
+        r = X::add(r, X::mul(X::mul(L::w(p), t.fac), S));
+      }
+      f[p] = r;
+    }
+  }
+  return odd;
+}
+
+// the functions above for one cell, a loop over the directions (cells that
+// collide64_cell gives back); stored: rho, u are given, else recovered with P
+template <class L>
+__device__ __noinline__ void collide64_redo(const double *fin, const int32_t *loff, double tau, bool stored,
+                                            const double *P, const double *F, double *state, double *out) {
+  double g[L::Q];
+#pragma unroll 1
+  for (int q = 0; q < L::Q; ++q) g[q] = fin[loff[q]];
+  double rho = state[0], u = state[1], v = state[2], w = state[3];
+  if (!stored) {
+    moments64<L>(g, P[0], P[1], P[2], rho, u, v, w);
+    if (L::D != 3) w = 0.0;
+  }
+  const bool hf = !(F[0] == 0.0 && F[1] == 0.0 && F[2] == 0.0);
+#pragma unroll 1
+  for (int q = 0; q < L::Q; ++q) {
+    const double cx = L::cx(q), cy = L::cy(q), cz = L::cz(q), wq = L::w(q);
+    out[q] = collide64v<L::D>(cx, cy, cz, wq, g[q], feq64v<L::D>(cx, cy, cz, wq, rho, u, v, w), tau, u, v, w,
+                              F[0], F[1], F[2], hf);
+  }
+}
+
 // shifted form (g = f - w): drho = rho - 1.  Every operation is an explicit
 // round-to-nearest intrinsic, so the result is the same in every kernel that
 // inlines it (no context-dependent contraction into FMA).

@@ -347,6 +347,7 @@ static int fill_args(const ilbm_ctx *ctx, const ilbm_box &b, const ilbm_level_pa
       a.fhi[d] = (d < D) ? std::min(p->force_hi[d], b.hi[d] + b.ngrow_m) : 0;
     }
     a.tau = p->tau;
+    a.tau64 = Tau64{p->tau, 1.0 / p->tau, 1.0 - 0.5 / p->tau};
     a.om32 = float(1.0 / p->tau);
     a.omh32 = float(1.0 - 0.5 / p->tau);
     a.self_fill = (p->ghost_mode == ILBM_GHOST_SELF);

@@ -313,14 +313,17 @@ __device__ __forceinline__ void step_cell(const StepArgs &a, int i, int j, int k
       v = ldm<double>(a.macro_in, m + 2 * a.ms2);
       w = (L::D == 3) ? ldm<double>(a.macro_in, m + 3 * a.ms2) : 0.0;
     } else {
-      moments64<L>(f, Px, Py, Pz, rho, u, v, w);
-      if (L::D != 3) w = 0.0;
+      moments64_fast<L>(f, Px, Py, Pz, rho, u, v, w);
     }
     // the Guo increment is skipped where F == 0 (collide_forced.H:81-83)
     const bool hf = ANY && !(Fx == R(0) && Fy == R(0) && Fz == R(0));
+    if (collide64_cell<L, ANY>(f, a.tau64, rho, u, v, w, Fx, Fy, Fz, hf)) {
+      const double Pd[3] = {Px, Py, Pz}, Fd[3] = {Fx, Fy, Fz};
+      double state[4] = {rho, u, v, w}, out[L::Q];
+      collide64_redo<L>(fin, a.loff, a.tau, ANY && stored, Pd, Fd, state, out);
 #pragma unroll
-    for (int q = 0; q < L::Q; ++q)
-      f[q] = collide64_one<L>(q, f[q], feq64<L>(q, rho, u, v, w), a.tau, u, v, w, Fx, Fy, Fz, hf);
+      for (int q = 0; q < L::Q; ++q) f[q] = out[q];
+    }
   } else {
     float drho, u, v, w;
     if (ANY && stored) {

@@ -6,6 +6,8 @@
 
 #include <stdint.h>
 
+#include "ilbm_common.cuh"
+
 namespace ilbm {
 
 constexpr int kMaxLevelBoxes = 64;
@@ -43,6 +45,7 @@ struct StepArgs {
   int bclo[3], bchi[3];
   double bvlo[3][4], bvhi[3][4];
   double tau;
+  Tau64 tau64;
   int self_fill;
   int use_uniform;
   double uf[3];
