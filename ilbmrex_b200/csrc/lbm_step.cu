@@ -48,13 +48,8 @@ int cuda_fail(cudaError_t e, const char *what) {
 // Macro pass (calculateMacroForcing) and equilibrium initialisation
 // ---------------------------------------------------------------------------
 template <class L, int S>
-__global__ void __launch_bounds__(256) k_macro(StepArgs a, int rlo0, int rlo1, int rlo2,
-                                               int rhi0, void *macro_out) {
+__device__ __forceinline__ void macro_cell(const StepArgs &a, int i, int j, int k, void *macro_out) {
   using R = typename Store<S>::R;
-  const int i = rlo0 + blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = rlo1 + blockIdx.y;
-  const int k = rlo2 + blockIdx.z;
-  if (i > rhi0) return;
   const int64_t base = fidx(a, i, j, k);
   R f[L::Q];
 #pragma unroll
@@ -78,6 +73,27 @@ __global__ void __launch_bounds__(256) k_macro(StepArgs a, int rlo0, int rlo1, i
     mo[m + 2 * a.ms2] = v;
     mo[m + 3 * a.ms2] = w;
   }
+}
+
+template <class L, int S>
+__global__ void __launch_bounds__(256) k_macro(StepArgs a, int rlo0, int rlo1, int rlo2,
+                                               int rhi0, void *macro_out) {
+  const int i = rlo0 + blockIdx.x * blockDim.x + threadIdx.x;
+  if (i <= rhi0) macro_cell<L, S>(a, i, rlo1 + blockIdx.y, rlo2 + blockIdx.z, macro_out);
+}
+
+// the macro pass of several boxes: box n's cells [rlo, rhi] start at block first[n]
+constexpr int kMacroThreads = 256;
+template <class L, int S>
+__global__ void __launch_bounds__(kMacroThreads) k_macro_boxes(const __grid_constant__ StepBoxes p) {
+  int n = 0;
+  while (n + 1 < p.nbox && blockIdx.x >= p.first[n + 1]) ++n;
+  const StepArgs &a = p.a[n];
+  const uint32_t c = (blockIdx.x - p.first[n]) * kMacroThreads + threadIdx.x;
+  if (c >= a.nvec) return;
+  const uint32_t row = fast_div(c, a.dvpr), kk = (L::D == 3) ? fast_div(row, a.dvny) : 0u;
+  macro_cell<L, S>(a, a.vx0 + (int)(c - row * a.vpr), a.rlo[1] + (int)(row - kk * a.vny), a.rlo[2] + (int)kk,
+                   p.macro_out[n]);
 }
 
 // InitEquilibrium, AmrCoreLBM.cpp:2117-2164, over the allocated f box
@@ -372,8 +388,8 @@ static int fill_args(const ilbm_ctx *ctx, const ilbm_box &b, const ilbm_level_pa
         return ILBM_ERR_RANGE;
       }
       a.nlb = p->nlevel_boxes;
-      for (int n = 0; n < a.nlb; ++n)
-        for (int c = 0; c < 6; ++c) a.lb[n][c] = p->level_boxes[6 * n + c];
+      if (a.nlb > 0)
+        for (int c = 0; c < 6; ++c) a.lb0[c] = p->level_boxes[c];
     }
   } else {
     a.f16_scale = scale16;
@@ -810,6 +826,94 @@ __global__ void __launch_bounds__(256) k_tags(TagArgs g, const R *vor, unsigned 
   if ((threadIdx.x & 31) == 0 && mine) atomicAdd(count, mine);
 }
 
+template <class L, int S>
+static int launch_boxes(ilbm_ctx *ctx, StepBoxes &p, const StepBoxes &whole) {
+  if (!launch_step_boxes<L, S>(ctx, p, ctx->stream)) {
+    // a very large box: one launch per box, with the level's boxes beside it
+    for (int n = 0; n < whole.nbox; ++n) {
+      StepBoxes one = whole;
+      one.nbox = 1;
+      one.a[0] = whole.a[n];
+      const int e = L::D - 1, last = one.a[0].rhi[e];
+      int64_t slice = 1;
+      for (int d = 0; d < e; ++d) slice *= one.a[0].rhi[d] - one.a[0].rlo[d] + 1;
+      const int most = (int)std::max<int64_t>(1, (int64_t)(1 << 26) / slice);
+      for (int s = one.a[0].rlo[e]; s <= last; s += most) {
+        one.a[0].rlo[e] = s;
+        one.a[0].rhi[e] = std::min(last, s + most - 1);
+        if (!launch_step_boxes<L, S>(ctx, one, ctx->stream)) {
+          set_error("box too large for one launch");
+          return ILBM_ERR_RANGE;
+        }
+        one.a[0].goff[3] = 0;  // the ghost shell goes with the first slice
+      }
+    }
+  }
+  return ILBM_OK;
+}
+
+template <class L, int S>
+static int launch_macro_boxes(ilbm_ctx *ctx, StepBoxes &p) {
+  uint32_t blocks = 0;
+  for (int n = 0; n < p.nbox; ++n) {
+    plan_vectors(p.a[n], L::D, 1);
+    p.first[n] = blocks;
+    blocks += (p.a[n].nvec + kMacroThreads - 1) / kMacroThreads;
+  }
+  p.first[p.nbox] = blocks;
+  if (blocks == 0) return ILBM_OK;
+  k_macro_boxes<L, S><<<blocks, kMacroThreads, 0, ctx->stream>>>(p);
+  ctx->launches++;
+  return ILBM_OK;
+}
+
+// the boxes of a level (caller-filled ghosts, checked): kMaxStepBoxes to a
+// launch, then their macro fields
+static int level_step_boxes(ilbm_ctx *ctx, const ilbm_box *boxes, int nbox, const ilbm_level_params *p) {
+  if (p->nlevel_boxes > kMaxLevelBoxes) {
+    set_error("level has more boxes than one call supports (64); split the call");
+    return ILBM_ERR_RANGE;
+  }
+  std::vector<StepBoxes> h(2);  // (the launch's parameters are too large for the stack to be pleasant)
+  StepBoxes &s = h[0], &m = h[1];
+  std::memset(&s, 0, sizeof(s));
+  for (int n = 0; n < p->nlevel_boxes; ++n)
+    for (int c = 0; c < 6; ++c) s.lb.lb[n][c] = p->level_boxes[6 * n + c];
+  for (int b0 = 0; b0 < nbox; b0 += kMaxStepBoxes) {
+    s.nbox = std::min(nbox - b0, kMaxStepBoxes);
+    int64_t cells = 0;
+    for (int n = 0; n < s.nbox; ++n) {
+      int rc = fill_args(ctx, boxes[b0 + n], p, s.a[n]);
+      if (rc) return rc;
+      int64_t c = 1;
+      for (int d = 0; d < ctx->dim; ++d) c *= s.a[n].rhi[d] - s.a[n].rlo[d] + 1;
+      cells = std::max(cells, c);
+    }
+    m = s;
+    int rc = ILBM_DISPATCH(ctx, launch_boxes, ctx, m, s);
+    if (rc) return rc;
+    m = s;
+    m.nbox = 0;
+    for (int n = 0; n < s.nbox; ++n) {
+      const ilbm_box &b = boxes[b0 + n];
+      if (!b.macro_out) continue;
+      if (cells > (1 << 26)) {  // as above: one launch per box
+        StepArgs am = s.a[n];
+        am.f_in = b.f_out;
+        if ((rc = ILBM_DISPATCH(ctx, launch_macro, ctx, am, am.rlo, am.rhi, b.macro_out))) return rc;
+        continue;
+      }
+      m.a[m.nbox] = s.a[n];
+      m.a[m.nbox].f_in = b.f_out;
+      m.macro_out[m.nbox++] = b.macro_out;
+    }
+    if (m.nbox > 0 && (rc = ILBM_DISPATCH(ctx, launch_macro_boxes, ctx, m))) return rc;
+  }
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return cuda_fail(e, "level step launch");
+  return ILBM_OK;
+}
+
 // one level step; with mlo / mhi the boxes' macro_in holds stored values
 // only on [mlo, mhi] (elsewhere rho, u are recovered from f^n and F^{n-1}),
 // and macro_out is written there only.  part (one box only): 0 = the whole
@@ -866,6 +970,10 @@ int level_step_impl(ilbm_ctx *ctx, const ilbm_box *boxes, int nbox, const ilbm_l
       set_error("f_in and f_out must be distinct (two-lattice scheme)");
       return ILBM_ERR_ARG;
     }
+  }
+  if (part == 0 && !mlo && (nbox > 1 || p->nlevel_boxes > 1)) return level_step_boxes(ctx, boxes, nbox, p);
+  for (int n = 0; n < nbox; ++n) {
+    const ilbm_box &b = boxes[n];
     StepArgs a;
     if ((rc = fill_args(ctx, b, p, a))) return rc;
     if (mlo && mhi) {

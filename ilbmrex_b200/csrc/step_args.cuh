@@ -74,8 +74,10 @@ struct StepArgs {
   // and the total (ghost_push)
   uint32_t goff[4];
   int face_lo[3], face_hi[3];  // what a face does with the populations that leave through it (FaceState)
+  // boxes of the level (caller-filled ghosts): their number and the first one;
+  // more come beside the arguments (LevelBoxes)
   int nlb;
-  int lb[kMaxLevelBoxes][6];
+  int lb0[6];
   // with use_mbox, macro_in holds stored values only on [mblo, mbhi]; cells
   // outside recover rho, u from f^n and F^{n-1}
   int use_mbox;
@@ -89,6 +91,23 @@ __device__ __forceinline__ bool stored_macro_at(const StepArgs &a, int i, int j,
   return i >= a.mblo[0] && i <= a.mbhi[0] && j >= a.mblo[1] && j <= a.mbhi[1] && k >= a.mblo[2] &&
          k <= a.mbhi[2];
 }
+
+// every box of a level (lo, hi), which decides whether a ghost cell is covered
+struct LevelBoxes {
+  int lb[kMaxLevelBoxes][6];
+};
+
+// The boxes of one launch of a level held in several boxes, passed by value
+// (so a captured launch owns them): box n's blocks start at first[n].
+constexpr int kMaxStepBoxes = 16;
+struct StepBoxes {
+  LevelBoxes lb;
+  int nbox;
+  uint32_t first[kMaxStepBoxes + 1];
+  void *macro_out[kMaxStepBoxes];
+  StepArgs a[kMaxStepBoxes];
+};
+static_assert(sizeof(StepBoxes) <= 32000, "kernel parameters hold at most 32,764 bytes");
 
 // One work item of the batched level step (k_step_batch): blockDim.x vectors
 // of case c from vector `first` on, or, with ghosts > 0, the ghost shell cells

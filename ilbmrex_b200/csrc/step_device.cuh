@@ -9,6 +9,11 @@
 
 namespace ilbm {
 
+// n / d by a multiplication (n < 2^31): d's magic from the host (div_magic)
+__device__ __forceinline__ uint32_t fast_div(uint32_t n, const DivMagic &d) {
+  return (__umulhi(n, d.mul) + n) >> d.shift;
+}
+
 __device__ __forceinline__ int64_t fidx(const StepArgs &a, int i, int j, int k) {
   return (int64_t)(i - a.fgl[0]) + (int64_t)(j - a.fgl[1]) * a.fs0 +
          (int64_t)(k - a.fgl[2]) * a.fs1;

@@ -29,6 +29,11 @@ int vec_width(const StepArgs &a);
 template <class L, int S>
 void launch_cells(ilbm_ctx *ctx, const StepArgs &a, cudaStream_t st, bool with_ghosts);
 
+// the boxes of a level (whole, with their ghost shells) in one launch; false,
+// with nothing launched: a box is too large for it
+template <class L, int S>
+bool launch_step_boxes(ilbm_ctx *ctx, StepBoxes &p, cudaStream_t st);
+
 // k_step_batch over a tile table, w threads per block
 template <class L, int S>
 int launch_step_batch(ilbm_ctx *ctx, const StepArgs *d_args, const StepTile *d_tiles, int ntiles, int V,
