@@ -700,8 +700,10 @@ __global__ void __launch_bounds__(1024) k_csr_scan(int n, int *rowptr, int cap, 
 __device__ __forceinline__ void csr_fill_row(const IBArgs &a, const double *xyz, double reg,
                                              const int *rowptr, int *col, double *val,
                                              double *diag, int i, int lane,
-                                             const double *tw = nullptr, const int4 *tc = nullptr) {
+                                             const double *tw = nullptr, const int4 *tc = nullptr,
+                                             double *rowmax = nullptr) {
   {
+    double sum = 0.0;
     int p = rowptr[i];
     for (int j0 = 0; j0 < a.n; j0 += 32) {
       const int j = j0 + lane;
@@ -712,9 +714,15 @@ __device__ __forceinline__ void csr_fill_row(const IBArgs &a, const double *xyz,
         const double v = tc ? ivc_entry_tab(a, tw, tc, i, j, reg) : ivc_entry(a, xyz, i, j, reg);
         col[slot] = j;
         val[slot] = v;
+        sum += fabs(v);
         if (i == j) diag[i] = v;
       }
       p += __popc(m);
+    }
+    if (rowmax) {  // the largest row sum (positive doubles order as integers)
+      for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if (lane == 0)
+        atomicMax(reinterpret_cast<unsigned long long *>(rowmax), (unsigned long long)__double_as_longlong(sum));
     }
   }
 }
@@ -723,12 +731,12 @@ __device__ __forceinline__ void csr_fill_row(const IBArgs &a, const double *xyz,
 __global__ void __launch_bounds__(256) k_csr_fill(IBArgs a, const double *xyz, double reg,
                                                   const int *rowptr, int *col, double *val,
                                                   double *diag, int cap, int *status,
-                                                  const double *tw, const int4 *tc) {
+                                                  const double *tw, const int4 *tc, double *rowmax) {
   if ((*status & 2) || rowptr[a.n] > cap) return;  // capacity exceeded (k_csr_scan)
   const int lane = threadIdx.x & 31;
   const int nw = (gridDim.x * blockDim.x) >> 5;
   for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < a.n; i += nw)
-    csr_fill_row(a, xyz, reg, rowptr, col, val, diag, i, lane, tw, tc);
+    csr_fill_row(a, xyz, reg, rowptr, col, val, diag, i, lane, tw, tc, rowmax);
 }
 
 // fixed-order reduction of per-block partials (nb blocks x 8 slots); every
@@ -981,16 +989,154 @@ __device__ __forceinline__ void cg_grid_body(cgrp::grid_group &grid, const IBArg
     for (int c = 0; c < 3; ++c) F[i + c * n] = X::add(F[i + c * n], X_[i + c * n]);
 }
 
+// The same systems by the Chebyshev iteration over the operator's known
+// spectrum: A = reg I + (a Gram matrix times dv > 0, IBMarkerDF.cpp:1106-1127),
+// so its eigenvalues lie in [reg, largest row sum] (about [1.3, 1.7] for
+// markers one cell apart, kChebMax the widest interval it is used on).  No
+// inner products: the residual of the k-th iterate is at most
+// |r0| / T_k((b + a) / (b - a)), which fixes the number of iterations once |r0|
+// is known, so a solve is one grid barrier per product and no reduction after
+// the first.  The vectors are held as (x, y, z, -) per marker, one 32-byte
+// sector per gathered column, and a row takes half a warp (97 entries: seven
+// rounds of 16 lanes instead of four of 32).  Bound by the latency of those L2
+// gathers beside the level step; CG took three products and six barriers for
+// the two iterations this needs two products and two barriers for:
+// the 12,869-marker sphere 104 -> 53 us per solve alone, the two-level sphere step
+// 719 -> 638 us.
+constexpr double kChebMax = 2.0;  // largest row sum / reg: the error falls by 5.8 or more per iteration
+
+__device__ __forceinline__ void half_row_dot(const int *col, const double *val, int e0, int e1, int hl,
+                                             const double *x4, double (&s)[3]) {
+  s[0] = s[1] = s[2] = 0.0;
+  for (int e = e0 + hl; e < e1; e += 64) {
+    int j[4];
+    double v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const bool on = e + 16 * u < e1;
+      j[u] = on ? col[e + 16 * u] : 0;
+      v[u] = on ? val[e + 16 * u] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const double2 xy = *reinterpret_cast<const double2 *>(x4 + 4 * (size_t)j[u]);
+      const double z = x4[4 * (size_t)j[u] + 2];
+      s[0] += v[u] * xy.x;
+      s[1] += v[u] * xy.y;
+      s[2] += v[u] * z;
+    }
+  }
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) s[c] += __shfl_xor_sync(0xffffffffu, s[c], o);
+}
+
+__device__ __forceinline__ void cheb_grid_body(cgrp::grid_group &grid, const IBArgs &a, const double *xyz,
+                                               const double *tgt, const double *uvw, const int *rowptr,
+                                               const int *col, const double *val, double lo, double hi,
+                                               double *X_, double *Xh, double *work, double *F, double *partial,
+                                               double tol, int *hist, int *iters, double (*sh)[8], double *red) {
+  const int n = a.n;
+  const int h = *hist, warm = h < 2 ? h : 2;
+  double *xa = work, *xb = work + 4 * (size_t)n, *D = work + 8 * (size_t)n, *B = work + 11 * (size_t)n;
+  const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gsz = gridDim.x * blockDim.x;
+  const int hl = gtid & 15, nh = gsz >> 4, gh = gtid >> 4;
+  const int rounds = (n + nh - 1) / nh;  // the same for every half warp: its shuffles stay convergent
+  for (int row = gh; row < n; row += nh)
+    if (hl < 3) {
+      const int e = row + hl * n;
+      const double xc = warm ? X_[e] : 0.0;
+      xa[4 * (size_t)row + hl] = warm >= 2 ? X::sub(X::mul(2.0, xc), Xh[e]) : xc;
+      if (warm) Xh[e] = xc;
+    }
+  grid.sync();
+  const double theta = 0.5 * (hi + lo), delta = fmax(0.5 * (hi - lo), 1.0e-9 * theta), s1 = theta / delta;
+  double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  for (int i = 0; i < rounds; ++i) {
+    const int row = gh + i * nh;
+    double s[3];
+    half_row_dot(col, val, row < n ? rowptr[row] : 0, row < n ? rowptr[row + 1] : 0, hl, xa, s);
+    if (row < n && hl < 3) {
+      double U[3];
+      target_of(a, row, xyz, tgt, U[0], U[1], U[2]);
+      const int e = row + hl * n;
+      const double b = X::div(X::sub(hl == 0 ? U[0] : (hl == 1 ? U[1] : U[2]), uvw[e]), a.dt);
+      const double r = b - (hl == 0 ? s[0] : (hl == 1 ? s[1] : s[2])), d = r / theta;
+      B[e] = b;
+      D[e] = d;
+      xb[4 * (size_t)row + hl] = xa[4 * (size_t)row + hl] + d;
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        if (hl == c) {
+          acc[c] += r * r;
+          acc[3 + c] += b * b;
+        }
+    }
+  }
+  block_partials(acc, 6, sh, partial);
+  grid.sync();
+  reduce_partials(partial, gridDim.x, 6, red);
+  // iterations: T_k(s1) >= |r0| / (tol |b|) for every component
+  double need = 1.0;
+  for (int c = 0; c < 3; ++c)
+    if (red[c] > 0.0) need = fmax(need, sqrt(red[c]) / (tol * sqrt(red[3 + c])));
+  int k = 1;
+  for (double t0 = 1.0, t1 = s1; t1 < need && k < 64; ++k) {
+    const double t2 = 2.0 * s1 * t1 - t0;
+    t0 = t1;
+    t1 = t2;
+  }
+  double rho = 1.0 / s1;
+  double *x = xb, *y = xa;
+  for (int it = 1; it < k; ++it) {
+    const double rn = 1.0 / (2.0 * s1 - rho), c1 = rn * rho, c2 = 2.0 * rn / delta;
+    rho = rn;
+    for (int i = 0; i < rounds; ++i) {
+      const int row = gh + i * nh;
+      double s[3];
+      half_row_dot(col, val, row < n ? rowptr[row] : 0, row < n ? rowptr[row + 1] : 0, hl, x, s);
+      if (row < n && hl < 3) {
+        const int e = row + hl * n;
+        const double d = c1 * D[e] + c2 * (B[e] - (hl == 0 ? s[0] : (hl == 1 ? s[1] : s[2])));
+        D[e] = d;
+        y[4 * (size_t)row + hl] = x[4 * (size_t)row + hl] + d;
+      }
+    }
+    double *const w = x;
+    x = y;
+    y = w;
+    if (it + 1 < k) grid.sync();
+  }
+  if (gtid == 0) {
+    *iters = k;
+    *hist = (h + 1 < 2) ? h + 1 : 2;
+  }
+  for (int row = gh; row < n; row += nh)
+    if (hl < 3) {
+      const int e = row + hl * n;
+      const double v = x[4 * (size_t)row + hl];
+      X_[e] = v;
+      F[e] = X::add(F[e], v);
+    }
+}
+
 __global__ void __launch_bounds__(256, 4) k_ivc_cg_grid(IBArgs a, const double *xyz, const double *tgt,
                                                      const double *uvw, const int *rowptr,
                                                      const int *col, const double *val,
                                                      const double *diag, double *X_, double *Xh,
                                                      double *work, double *F, double *partial,
                                                      int maxit, double tol, int *hist, int *status,
-                                                     int *iters) {
+                                                     int *iters, double reg, const double *rowmax) {
   cgrp::grid_group grid = cgrp::this_grid();
   __shared__ double sh[8][8];
   __shared__ double red[8];
+  const double hi = *rowmax * (1.0 + 1.0e-12);  // (the same for every block: a uniform branch)
+  if (reg > 0.0 && a.dv > 0.0 && hi <= kChebMax * reg) {
+    cheb_grid_body(grid, a, xyz, tgt, uvw, rowptr, col, val, reg, hi, X_, Xh, work, F, partial, tol, hist,
+                   iters, sh, red);
+    return;
+  }
   cg_grid_body(grid, a, xyz, tgt, uvw, rowptr, col, val, diag, X_, Xh, work, F, partial, maxit, tol,
                hist, status, iters, sh, red);
 }
@@ -1856,6 +2002,7 @@ struct ilbm_ib {
   int nnz_cap = 0;
   bool csr_ready = false;
   double *d_partial = nullptr;  // CG block partials
+  double *d_rowmax = nullptr;   // the operator's largest row sum (bounds its spectrum from above)
   int cg_blocks = 0;
   // the IVC solutions the next CG start may use (device int, 0-2): d_X the
   // last, d_Xh the one before it; the solves themselves advance it
@@ -2311,7 +2458,7 @@ int ilbm_ib_create(ilbm_ctx *ctx, const ilbm_ib_params *p, const ilbm_level_geom
     if ((rc = dmalloc(ib, &ib->d_rowptr, (size_t)n + 1)) || (rc = dmalloc(ib, &ib->d_col, (size_t)ib->nnz_cap)) ||
         (rc = dmalloc(ib, &ib->d_val, (size_t)ib->nnz_cap)) || (rc = dmalloc(ib, &ib->d_diag, (size_t)n)) ||
         (rc = dmalloc(ib, &ib->d_X, 3 * (size_t)n)) || (rc = dmalloc(ib, &ib->d_Xh, 3 * (size_t)n)) ||
-        (rc = dmalloc(ib, &ib->d_hist, 1)) ||
+        (rc = dmalloc(ib, &ib->d_hist, 1)) || (rc = dmalloc(ib, &ib->d_rowmax, 1)) ||
         (rc = dmalloc(ib, &ib->d_work, 15 * (size_t)n)) ||
         (rc = dmalloc(ib, &ib->d_tw, (size_t)kTabStride * n)) || (rc = dmalloc(ib, &ib->d_tc, (size_t)n))) {
       ilbm_ib_destroy(ib);
@@ -2406,8 +2553,10 @@ static int launch_cg(ilbm_ib *ib, const IBArgs &a_in, cudaStream_t s) {
   int maxit = 500;
   double tol = cg_tol;
   int *hist = ib->d_hist, *status = ib->d_status, *iters = ib->d_iters;
+  double reg = ib->p.ivc_diag_reg;
+  const double *rowmax = ib->d_rowmax;
   void *args[] = {&a, &xyz, &tgt, &uvw, &rowptr, &col, &val, &diag, &Xv, &Xh, &work, &Fm,
-                  &partial, &maxit, &tol, &hist, &status, &iters};
+                  &partial, &maxit, &tol, &hist, &status, &iters, &reg, &rowmax};
   // one warp per ~2 rows keeps the SpMV latency-tolerant; more blocks than
   // that only make the grid barriers dearer
   const int blocks = std::max(8, std::min(ib->cg_blocks, (ib->n + 15) / 16));
@@ -2606,9 +2755,11 @@ static int ib_update(ilbm_ib *ib, const ilbm_box *boxes, int nbox, const ilbm_le
       if (!ib->csr_ready || ib->moving || ib->p.ivc_rebuild_matrix > 0) {
         const int cb = std::min(4096, (ib->n * 32 + 255) / 256);
         k_csr_count<<<cb, 256, 0, s>>>(a, ib->d_xyz, ib->d_rowptr, tc);
+        cudaMemsetAsync(ib->d_rowmax, 0, sizeof(double), s);
         k_csr_scan<<<1, 1024, 0, s>>>(ib->n, ib->d_rowptr, ib->nnz_cap, ib->d_status);
         k_csr_fill<<<cb, 256, 0, s>>>(a, ib->d_xyz, ib->p.ivc_diag_reg, ib->d_rowptr, ib->d_col,
-                                      ib->d_val, ib->d_diag, ib->nnz_cap, ib->d_status, tw, tc);
+                                      ib->d_val, ib->d_diag, ib->nnz_cap, ib->d_status, tw, tc,
+                                      ib->d_rowmax);
         ctx->launches += 3;
         ib->csr_ready = true;
       }
