@@ -466,7 +466,7 @@ static int launch_step_split(ilbm_ctx *ctx, const StepArgs &a, const int *blo, c
     inner.rlo[d] = blo[d];
     inner.rhi[d] = bhi[d];
   }
-  launch_cells<L, S>(ctx, inner, ctx->stream, false);
+  launch_cells<L, S>(ctx, inner, ctx->stream, false, true);
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "level step launch");
   return ILBM_OK;

@@ -25,9 +25,10 @@ bool plan_vectors(StepArgs &a, int dim, int V);
 template <class L, int S>
 int vec_width(const StepArgs &a);
 
-// k_step over [rlo, rhi] (minus the skip box), with the ghost shell push or not
+// k_step over [rlo, rhi] (minus the skip box), with the ghost shell push or
+// not; singly: in the cell form whatever the layout
 template <class L, int S>
-void launch_cells(ilbm_ctx *ctx, const StepArgs &a, cudaStream_t st, bool with_ghosts);
+void launch_cells(ilbm_ctx *ctx, const StepArgs &a, cudaStream_t st, bool with_ghosts, bool singly = false);
 
 // the boxes of a level (whole, with their ghost shells) in one launch; false,
 // with nothing launched: a box is too large for it
