@@ -51,6 +51,7 @@ using namespace ilbm;
 // (ib_chain.cuh) bodies whose forcing chain is one launch
 static constexpr int kChainMaxMarkers = 512, kChainMaxCg = 448;
 static constexpr int64_t kChainMaxBand = 65536;
+static constexpr size_t kChainSharedMax = 224 * 1024;  // dynamic shared memory of a block
 
 namespace {
 
@@ -404,17 +405,19 @@ __device__ __forceinline__ bool may_couple_tab(const IBArgs &a, const int4 *tc, 
   return abs(ci.x - cj.x) <= 4 && abs(ci.y - cj.y) <= 4 && (a.dim < 3 || abs(ci.z - cj.z) <= 4);
 }
 __device__ double ivc_entry_tab(const IBArgs &a, const double *tw, const int4 *tc, int i, int j,
-                                double reg) {
+                                double reg, int stride = kTabStride) {
   const int4 ci = tc[i], cj = tc[j];
-  const double *wi = tw + (int64_t)kTabStride * i, *wj = tw + (int64_t)kTabStride * j;
+  const double *wi = tw + (int64_t)stride * i, *wj = tw + (int64_t)stride * j;
   auto overlap = [&](int d) {
     const int ia = tab_cell(ci, d), ib = tab_cell(cj, d);
-    int lo = max(ia - 2, ib - 2), hi = min(ia + 2, ib + 2);
-    lo = max(lo, a.dlo[d]);
-    hi = min(hi, a.dhi[d]);
-    double sum = 0.0;  // stays 0 when lo > hi, as overlap_1d
-    for (int q = lo; q <= hi; ++q)
-      sum = X::add(sum, X::mul(X::mul(wi[5 * d + q - ia + 2], wj[5 * d + q - ib + 2]), a.dx[d]));
+    double sum = 0.0;  // stays 0 when no cell is shared, as overlap_1d
+#pragma unroll
+    for (int o = 0; o < 5; ++o) {  // (unrolled: the loads of all five cells in flight)
+      const int q = ia + o - 2, p = q - ib + 2;
+      const bool on = p >= 0 && p < 5 && q >= a.dlo[d] && q <= a.dhi[d];
+      const double t = on ? X::mul(X::mul(wi[5 * d + o], wj[5 * d + p]), a.dx[d]) : 0.0;
+      sum = X::add(sum, t);
+    }
     return sum;
   };
   const double sx = overlap(0), sy = overlap(1), sz = (a.dim == 3) ? overlap(2) : 1.0;
@@ -2382,6 +2385,8 @@ int enable_dense(ilbm_ib *ib) {
 
 }  // namespace
 
+static int chain_prepare(ilbm_ctx *ctx);
+
 extern "C" {
 
 int ilbm_ib_create(ilbm_ctx *ctx, const ilbm_ib_params *p, const ilbm_level_geom *g,
@@ -2481,6 +2486,10 @@ int ilbm_ib_create(ilbm_ctx *ctx, const ilbm_ib_params *p, const ilbm_level_geom
       ilbm_ib_destroy(ib);
       return rc;
     }
+  }
+  if ((rc = chain_prepare(ctx))) {
+    ilbm_ib_destroy(ib);
+    return rc;
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
@@ -3136,44 +3145,17 @@ struct IBCase {
   int gcells;
 };
 
-#include "ib_chain.cuh"
-
 // a case that has taken all the steps it was added for sits out
 __device__ __forceinline__ bool live(const int *steps, const int *limit, int c) {
   return steps[c] < limit[c];
 }
 
-__global__ void __launch_bounds__(256) k_b_markers(const IBCase *cs, const ItemRef *list, int64_t cnt,
-                                                   const int *steps, const int *limit) {
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < cnt;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const ItemRef e = list[t];
-    const int c = e.c;
-    if (!live(steps, limit, c)) continue;
-    const IBCase &k = cs[c];
-    const int m = e.u;
-    if (m == 0) {
-      k.fsum[0] = k.fsum[1] = k.fsum[2] = 0.0;
-      k.status[0] = 0;
-    }
-    double kc = 1.0, ks = 0.0, om = 0.0;
-    if (k.moving) {
-      int s = steps[c];
-      if (s >= k.kin_steps) {
-        if (m == 0) atomicOr(k.status, 16);  // ran past its kinematics table
-        s = k.kin_steps - 1;
-      }
-      om = k.kin[4 * s];
-      kc = k.kin[4 * s + 1];
-      ks = k.kin[4 * s + 2];
-    }
-    markers_one(k.a, kc, ks, om, m, k.xyz, k.ref, k.tgt, k.uvw, k.F);
-  }
-}
+#include "ib_chain.cuh"
 
-// one block of kItemTile threads per band tile
+// SumBoundary of the bands that reach over a periodic face, one block of
+// kItemTile threads per band tile
 __global__ void __launch_bounds__(kItemTile) k_b_band(const IBCase *cs, const ItemRef *tiles, int ntiles,
-                                                      int op, const int *steps, const int *limit) {
+                                                      const int *steps, const int *limit) {
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const ItemRef e = tiles[t];
     const int c = e.c;
@@ -3181,21 +3163,12 @@ __global__ void __launch_bounds__(kItemTile) k_b_band(const IBCase *cs, const It
     const IBCase &k = cs[c];
     const int64_t u = (int64_t)e.u + threadIdx.x;
     if (u >= k.a.nb) continue;
-    if (op == 0) {
-      k.EFI[u] = 0.0;
-      k.EFI[u + k.a.nb] = 0.0;
-      k.EFI[u + 2 * k.a.nb] = 0.0;
-    } else if (op == 1) {
-      if (k.periodic_band) fill_boundary_cell(k.a, k.EV, u);
-    } else {
-      if (k.periodic_band) sum_boundary_cell(k.a, k.EFI, u);
-    }
+    if (k.periodic_band) sum_boundary_cell(k.a, k.EFI, u);
   }
 }
 
-// one warp per marker; stage 0 interpolation (writes the weight table), 1
-// explicit force, 2 spreading, 3 CSR row count, 4 CSR row fill (2-4 read the
-// table)
+// one warp per marker; stage 1 explicit force, 2 spreading, 3 CSR row count, 4
+// CSR row fill (2-4 read the interpolation's weight table)
 template <int stage>
 __global__ void __launch_bounds__(128) k_b_marker_warp(const IBCase *cs, const ItemRef *list, int64_t cnt,
                                                        const int *steps, const int *limit) {
@@ -3207,10 +3180,7 @@ __global__ void __launch_bounds__(128) k_b_marker_warp(const IBCase *cs, const I
     if (!live(steps, limit, c)) continue;
     const IBCase &k = cs[c];
     const int m = e.u;
-    if constexpr (stage == 0) {
-      interp_one(k.a, m, lane, k.xyz, k.EV, k.uvw, k.status, k.tgt, k.mode == 1 ? k.rhs : nullptr,
-                 k.ld, k.tw, k.tc);
-    } else if constexpr (stage == 1) {
+    if constexpr (stage == 1) {
       if (k.mode == 0 && lane == 0) force_explicit_one(k.a, m, k.xyz, k.tgt, k.uvw, k.F);
     } else if constexpr (stage == 2) {
       spread_one_tab(k.a, m, lane, k.tw, k.tc, k.F, k.EFI, k.status);
@@ -3253,25 +3223,50 @@ __global__ void __launch_bounds__(kDenseThreads) k_b_dense(const IBCase *cs, con
     dense_row(k.a, k.rhs, k.Ainv, k.ld, k.F, e.u);
 }
 
-template <class R>
-// each tile also leaves the fixed-order sum of the force it stored (tpart,
-// 3 per tile): the case's Eulerian force sum, combined by k_b_record
+// F = dt rho a over the band (rho formed where a force was spread, zero
+// elsewhere); the spread force is left zero for the next step.  Each tile also
+// leaves the fixed-order sum of the force it stored (tpart, 3 per tile): the
+// case's Eulerian force sum, combined by k_b_record
+template <class L, int S>
 __global__ void __launch_bounds__(kItemTile) k_b_export(const IBCase *cs, const ItemRef *tiles,
                                                         int ntiles, const StepArgs *args,
                                                         const int *steps, const int *limit,
                                                         double *tpart) {
+  using R = typename Store<S>::R;
   __shared__ double shr[kMaxWarps][3];
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const ItemRef e = tiles[t];
     const int c = e.c;
     if (!live(steps, limit, c)) continue;  // uniform over the block
     const IBCase &k = cs[c];
+    const IBArgs &a = k.a;
     const int64_t u = (int64_t)e.u + threadIdx.x;
     double v[3] = {0.0, 0.0, 0.0};
-    if (u < k.a.nb) {
+    if (u < a.nb) {
       const StepArgs &sa = args[c];
-      export_cell<R>(k.a, k.EFI, k.RHO, static_cast<R *>(const_cast<void *>(sa.force)), sa.mgl[0],
-                     sa.mgl[1], sa.mgl[2], sa.ms0, sa.ms1, sa.ms2, u, v);
+      const double f[3] = {k.EFI[u], k.EFI[u + a.nb], a.dim == 3 ? k.EFI[u + 2 * a.nb] : 0.0};
+      const uint32_t w = (uint32_t)u, r = w / (uint32_t)a.bn[0];  // (a band has fewer than 2^31 cells)
+      const int i = a.blo[0] + (int)(w - r * (uint32_t)a.bn[0]);
+      const int q = a.dim == 3 ? (int)(r / (uint32_t)a.bn[1]) : 0, j = a.blo[1] + (int)r - q * a.bn[1];
+      const int kz = a.dim == 3 ? a.blo[2] + q : 0;
+      const bool some = f[0] != 0.0 || f[1] != 0.0 || f[2] != 0.0;
+      if (i >= a.dlo[0] && i <= a.dhi[0] && j >= a.dlo[1] && j <= a.dhi[1] &&
+          (a.dim == 2 || (kz >= a.dlo[2] && kz <= a.dhi[2]))) {
+        double dr = 0.0;
+        if (some) {
+          double m4[4];
+          band_macro_value<L, S>(sa, i, j, kz, m4);
+          dr = X::mul(a.dt, m4[0]);
+        }
+        R *F = static_cast<R *>(const_cast<void *>(sa.force));
+        const int64_t m = midx(sa, i, j, kz);
+        for (int d = 0; d < a.dim; ++d) {
+          const R x = R(X::mul(dr, f[d]));
+          F[m + d * sa.ms2] = x;
+          v[d] = double(x);
+        }
+      }
+      if (some) k.EFI[u] = k.EFI[u + a.nb] = k.EFI[u + 2 * a.nb] = 0.0;
     }
     double tot[3];
     block_reduce<3>(v, shr, tot);
@@ -3359,16 +3354,23 @@ static void chain_case(ilbm_ib *ib, const IBArgs &a, int mode, IBCase &k) {
   }
 }
 
+// what the chain kernel's launches need, once per body (on the body's device)
 template <class L, int S>
-static int launch_chain_of(ilbm_ctx *ctx, const ChainArgs &c, cudaStream_t s) {
+static int chain_prepare_of(ilbm_ctx *) {
   cudaError_t e = cudaFuncSetAttribute(k_ib_chain<L, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)chain_shared(2, kChainMaxCg));
+                                       (int)chain_shared(2, kChainMaxCg, 3));
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_ib_chain<L, S>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e != cudaSuccess) return cuda_fail(e, "body forcing: shared memory");
-  k_ib_chain<L, S><<<kChainCtas, kChainThreads, chain_shared(c.k.mode, c.k.a.n), s>>>(c);
+  return ILBM_OK;
+}
+static int chain_prepare(ilbm_ctx *ctx) { return ILBM_DISPATCH(ctx, chain_prepare_of, ctx); }
+
+template <class L, int S>
+static int launch_chain_of(ilbm_ctx *ctx, const ChainArgs &c, cudaStream_t s) {
+  k_ib_chain<L, S><<<kChainCtas, kChainThreads, chain_shared(c.k.mode, c.k.a.n, c.k.a.dim), s>>>(c);
   ctx->launches++;
-  e = cudaGetLastError();
+  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "body forcing");
   return ILBM_OK;
 }
@@ -3395,7 +3397,6 @@ struct IBBatch {
   int nc = 0, rec_slots = 1;
   std::vector<void *> allocs;
   IBCase *d_cases = nullptr;
-  BandDesc *d_bands = nullptr;
   int64_t total_m = 0, total_b = 0, total_drows = 0, total_rm = 0;
   int nbt = 0;  // band tiles
   // work lists: every marker, the markers of bodies whose operator is
@@ -3404,6 +3405,10 @@ struct IBBatch {
   ItemRef *d_mlist = nullptr, *d_rlist = nullptr, *d_dlist = nullptr, *d_btiles = nullptr;
   int *d_cgcase = nullptr;
   int ncg = 0;
+  // rebuilding bodies whose rows fit a cluster's shared memory (k_b_cluster_cg)
+  int *d_clcase = nullptr;
+  int ncl = 0;
+  size_t cl_shared = 0;
   bool any_periodic = false, any_explicit = false, any_rebuild = false;
   int *d_steps = nullptr, *d_limit = nullptr;
   double *d_rec = nullptr, *d_tpart = nullptr;  // record rings; the export's tile partials
@@ -3456,6 +3461,8 @@ int ib_batch_create(ilbm_ctx *ctx, const std::vector<IBBatchCase> &cases, int re
   {
     cudaError_t e = cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k_b_cluster_cg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChainSharedMax);
     if (e != cudaSuccess) {
       ib_batch_destroy(b);
       return cuda_fail(e, "IB batch events");
@@ -3464,16 +3471,13 @@ int ib_batch_create(ilbm_ctx *ctx, const std::vector<IBBatchCase> &cases, int re
   b->nc = (int)cases.size();
   b->rec_slots = std::max(1, rec_slots);
   std::vector<IBCase> hc(b->nc);
-  std::vector<BandDesc> hb(b->nc);
   std::vector<int64_t> moff(b->nc + 1, 0), boff(b->nc + 1, 0);
-  std::vector<int> cgcase;
+  std::vector<int> cgcase, clcase;
   std::vector<ItemRef> mlist, rlist, dlist, btiles;
   std::vector<std::vector<double>> kin(b->nc);
   for (int c = 0; c < b->nc; ++c) {
     IBCase &k = hc[c];
     std::memset(&k, 0, sizeof(k));
-    BandDesc &bd = hb[c];
-    std::memset(&bd, 0, sizeof(bd));
     ilbm_ib *ib = cases[c].ib;
     moff[c + 1] = moff[c];
     boff[c + 1] = boff[c];
@@ -3523,6 +3527,7 @@ int ib_batch_create(ilbm_ctx *ctx, const std::vector<IBBatchCase> &cases, int re
     k.hist = ib->d_hist;
     k.work = ib->d_work;
     k.nnz_cap = ib->nnz_cap;
+    if (ib->gather && ib->sw_ready) k.sw = static_cast<const SpreadW *>(ib->d_sw);
     k.reg = ib->p.ivc_diag_reg;
     k.cg_tol = ivc_cg_tolerance(ctx->storage);
     k.Ainv = ib->d_Ainv;
@@ -3548,23 +3553,23 @@ int ib_batch_create(ilbm_ctx *ctx, const std::vector<IBBatchCase> &cases, int re
     }
     moff[c + 1] = moff[c] + ib->n;
     boff[c + 1] = boff[c] + ib->nb;
+    const bool cluster = k.mode == 2 && k.rebuild && chain_shared(2, ib->n, ib->dim, kBatchCgCtas) <= kChainSharedMax;
     for (int m = 0; m < ib->n; ++m) {
       mlist.push_back({c, m});
-      if (k.rebuild) rlist.push_back({c, m});
+      if (k.rebuild && !cluster) rlist.push_back({c, m});
       if (k.mode == 1) dlist.push_back({c, m});
     }
     k.tile0 = (int)btiles.size();
     for (int64_t u = 0; u < ib->nb; u += kItemTile) btiles.push_back({c, (int)u});
     k.ntile = (int)btiles.size() - k.tile0;
-    for (int d = 0; d < 3; ++d) {
-      bd.blo[d] = ib->blo[d];
-      bd.bn[d] = ib->bn[d];
+    if (cluster) {
+      clcase.push_back(c);
+      b->cl_shared = std::max(b->cl_shared, chain_shared(2, ib->n, ib->dim, kBatchCgCtas));
+    } else if (k.mode == 2) {
+      cgcase.push_back(c);
     }
-    bd.nb = ib->nb;
-    bd.EV = ib->d_EV;
-    bd.RHO = ib->d_RHO;
-    bd.EFI = ib->d_EFI;
-    if (k.mode == 2) cgcase.push_back(c);
+    // zero on entry of every step, as the export leaves it
+    cudaMemsetAsync(ib->d_EFI, 0, 3 * (size_t)ib->nb * sizeof(double), ctx->stream);
     b->any_periodic = b->any_periodic || k.periodic_band;
     b->any_explicit = b->any_explicit || k.mode == 0;
     b->any_rebuild = b->any_rebuild || k.rebuild;
@@ -3614,10 +3619,11 @@ int ib_batch_create(ilbm_ctx *ctx, const std::vector<IBBatchCase> &cases, int re
   b->total_rm = (int64_t)rlist.size();
   b->nbt = (int)btiles.size();
   b->ncg = (int)cgcase.size();
-  if ((rc = bupload(b, &b->d_cases, hc)) || (rc = bupload(b, &b->d_bands, hb)) ||
+  b->ncl = (int)clcase.size();
+  if ((rc = bupload(b, &b->d_cases, hc)) ||
       (rc = bupload(b, &b->d_mlist, mlist)) || (rc = bupload(b, &b->d_rlist, rlist)) ||
       (rc = bupload(b, &b->d_dlist, dlist)) || (rc = bupload(b, &b->d_btiles, btiles)) ||
-      (rc = bupload(b, &b->d_cgcase, cgcase))) {
+      (rc = bupload(b, &b->d_cgcase, cgcase)) || (rc = bupload(b, &b->d_clcase, clcase))) {
     ib_batch_destroy(b);
     return rc;
   }
@@ -3630,33 +3636,43 @@ int ib_batch_create(ilbm_ctx *ctx, const std::vector<IBBatchCase> &cases, int re
   return ILBM_OK;
 }
 
+template <class L, int S>
+static int launch_b_interp(ilbm_ctx *ctx, IBBatch *b, const StepArgs *d_args, int blocks, cudaStream_t s) {
+  k_b_interp<L, S><<<blocks, 128, 0, s>>>(b->d_cases, d_args, b->d_mlist, b->total_m, b->d_steps, b->d_limit);
+  ctx->launches++;
+  return ILBM_OK;
+}
+
+template <class L, int S>
+static int launch_b_export(ilbm_ctx *ctx, IBBatch *b, const StepArgs *d_args, int blocks, cudaStream_t s) {
+  k_b_export<L, S><<<blocks, kItemTile, 0, s>>>(b->d_cases, b->d_btiles, b->nbt, d_args, b->d_steps, b->d_limit,
+                                                b->d_tpart);
+  ctx->launches++;
+  return ILBM_OK;
+}
+
 int ib_batch_forcing(IBBatch *b, const StepArgs *d_args, cudaStream_t s) {
   ilbm_ctx *ctx = b->ctx;
   if (b->total_m == 0) return ILBM_OK;
   const int *st = b->d_steps, *lm = b->d_limit;
-  int rc = batch_band_macro_launch(ctx, d_args, b->d_bands, b->d_btiles, b->nbt, st, lm, s);
-  if (rc) return rc;
-  const int gt = std::min(b->nbt, 4096), gm = grid_for(b->total_m, 256);
+  const int gt = std::min(b->nbt, 4096);
   const int gw = grid_for(b->total_m * 32, 128), gr = grid_for(b->total_rm * 32, 128);
   const ItemRef *ml = b->d_mlist, *rl = b->d_rlist;
   const int64_t nm = b->total_m, nr = b->total_rm;
-  // (the band macro also zeroed EFI)
-  k_b_markers<<<gm, 256, 0, s>>>(b->d_cases, ml, nm, st, lm);
-  ctx->launches += 1;
-  if (b->any_periodic) {
-    k_b_band<<<gt, kItemTile, 0, s>>>(b->d_cases, b->d_btiles, b->nbt, 1, st, lm);
-    ctx->launches++;
-  }
-  k_b_marker_warp<0><<<gw, 128, 0, s>>>(b->d_cases, ml, nm, st, lm);
-  ctx->launches++;
+  int rc = ILBM_DISPATCH(ctx, launch_b_interp, ctx, b, d_args, gw, s);
+  if (rc) return rc;
   // the moving bodies' operator build and CG (the longer chain) on the
   // high-priority side stream, the stored-inverse solves beside them
-  const bool fork = b->ncg > 0 && b->total_drows > 0;
+  const bool fork = b->ncg + b->ncl > 0 && b->total_drows > 0;
   cudaStream_t cgs = fork ? ctx->side : s;
   if (fork) {
     cudaError_t e = cudaEventRecord(b->ev_fork, s);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(cgs, b->ev_fork, 0);
     if (e != cudaSuccess) return cuda_fail(e, "batched IVC fork");
+  }
+  if (b->ncl > 0) {
+    k_b_cluster_cg<<<b->ncl * kBatchCgCtas, kChainThreads, b->cl_shared, cgs>>>(b->d_cases, b->d_clcase, st, lm);
+    ctx->launches++;
   }
   if (nr > 0) {
     k_b_marker_warp<3><<<gr, 128, 0, cgs>>>(b->d_cases, rl, nr, st, lm);
@@ -3684,16 +3700,10 @@ int ib_batch_forcing(IBBatch *b, const StepArgs *d_args, cudaStream_t s) {
   k_b_marker_warp<2><<<gw, 128, 0, s>>>(b->d_cases, ml, nm, st, lm);
   ctx->launches++;
   if (b->any_periodic) {
-    k_b_band<<<gt, kItemTile, 0, s>>>(b->d_cases, b->d_btiles, b->nbt, 2, st, lm);
+    k_b_band<<<gt, kItemTile, 0, s>>>(b->d_cases, b->d_btiles, b->nbt, st, lm);
     ctx->launches++;
   }
-  if (ctx->storage == ILBM_STORAGE_F64)
-    k_b_export<double><<<gt, kItemTile, 0, s>>>(b->d_cases, b->d_btiles, b->nbt, d_args, st, lm,
-                                                 b->d_tpart);
-  else
-    k_b_export<float><<<gt, kItemTile, 0, s>>>(b->d_cases, b->d_btiles, b->nbt, d_args, st, lm,
-                                                b->d_tpart);
-  ctx->launches++;
+  if ((rc = ILBM_DISPATCH(ctx, launch_b_export, ctx, b, d_args, gt, s))) return rc;
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "batched update_forcing");
   return ILBM_OK;

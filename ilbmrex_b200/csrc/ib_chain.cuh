@@ -34,10 +34,15 @@ constexpr int kChainThreads = 512;
 // A, z and p of every marker, x, r, Ap, b and diagonal of its own rows, the
 // reduction slots, the markers' weights and cells; stored inverse: the
 // right-hand side
-__host__ __device__ inline size_t chain_shared(int mode, int n) {
-  const size_t rows = (size_t)(n + kChainCtas - 1) / kChainCtas;
+// a marker's weights in shared memory: an odd stride, so that consecutive
+// markers' weights lie in different banks (stride 16 made every read of the
+// operator's build a 32-way conflict: 77 -> 73 us of a 32-case batch step)
+__host__ __device__ constexpr int chain_stride(int dim) { return 5 * dim + (dim == 2 ? 1 : 2); }
+__host__ __device__ inline size_t chain_shared(int mode, int n, int dim, int ctas = kChainCtas) {
+  const size_t rows = (size_t)(n + ctas - 1) / ctas;
   if (mode == 2)
-    return (rows * n + 6 * (size_t)n + 13 * rows + 2 * kChainCtas * 6 + 8 + (kTabStride + 2) * (size_t)n) * sizeof(double);
+    return (rows * n + 6 * (size_t)n + 13 * rows + 2 * (size_t)ctas * 6 + 8 + (chain_stride(dim) + 2) * (size_t)n) *
+           sizeof(double);
   return mode == 1 ? 3 * (size_t)n * sizeof(double) : 0;
 }
 
@@ -152,93 +157,127 @@ __device__ __forceinline__ void chain_dense_row(const IBCase &k, const TA *Ainv,
 }
 
 // Jacobi-preconditioned CG (ivc_cg_block's iteration) over the cluster: block
-// `rank` owns rows [r0, r1) as dense rows of A in its shared memory.  Every
-// block holds z and p of all markers; a block's z rows and partial sums go to
-// all blocks through distributed shared memory, and each sums the
-// partials in the same order, so all blocks take the same branches.
-template <class L>
+// `rank` owns rows [r0, r0 + nl) as dense rows of A in its shared memory, up to
+// four consecutive ones per warp.  A product reads a column's p once for a
+// warp's rows and skips the 32-column chunks none of them couples to (a marker
+// couples within four cells, 60-100 of 384 columns): with a row at a time over
+// all columns the loads of p from shared memory alone took 3,500 cycles per
+// product of 48 rows.  Every block holds z and p of all markers; a block's z
+// rows and partial sums go to all blocks through distributed shared memory, and
+// each sums the partials in the same order, so all blocks take the same branches.
+template <int CTAS>
 __device__ __forceinline__ void chain_cg(cgrp::cluster_group &cl, const IBCase &k, const IBArgs &a, double *sh) {
+  constexpr int NW = kChainThreads / 32, RW = 4;
   const int n = a.n, rank = (int)cl.block_rank(), tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int nw = kChainThreads / 32;
-  const int rows = (n + kChainCtas - 1) / kChainCtas, r0 = min(n, rank * rows), nl = min(n, r0 + rows) - r0;
+  const int rows = (n + CTAS - 1) / CTAS, r0 = min(n, rank * rows), nl = min(n, r0 + rows) - r0;
   int4 *tc = reinterpret_cast<int4 *>(sh);  // first: 16-byte aligned whatever n is
-  double *tw = sh + 2 * (size_t)n, *A = tw + (size_t)kTabStride * n, *z = A + (size_t)rows * n, *p = z + 3 * n;
+  const int ws = chain_stride(a.dim);
+  double *tw = sh + 2 * (size_t)n, *A = tw + (size_t)ws * n, *z = A + (size_t)rows * n, *p = z + 3 * n;
   double *x = p + 3 * n, *r = x + 3 * rows, *ap = r + 3 * rows, *b = ap + 3 * rows, *dg = b + 3 * rows;
-  double *slot = dg + rows;  // [2][kChainCtas][6]
-  double *tot = slot + 2 * kChainCtas * 6;
-  // the operator's rows from the step's weight table
-  for (int t = tid; t < kTabStride * n; t += kChainThreads) tw[t] = k.tw[t];
+  double *slot = dg + rows;  // [2][CTAS][6]
+  double *tot = slot + 2 * CTAS * 6;
+  // the step's weight table, and the start: zero, the last solution, or the
+  // extrapolation of the last two
+#pragma unroll 4
+  for (int t = tid; t < kTabStride * n; t += kChainThreads) {
+    const double v = k.tw[t];
+    if (t % kTabStride < 5 * a.dim) tw[t / kTabStride * ws + t % kTabStride] = v;
+  }
   for (int t = tid; t < n; t += kChainThreads) tc[t] = k.tc[t];
-  __syncthreads();
-  for (int i = wid; i < nl; i += nw)
-    for (int j = lane; j < n; j += 32) {
-      const int row = r0 + i;
-      const double v = may_couple_tab(a, tc, row, j) ? ivc_entry_tab(a, tw, tc, row, j, k.reg) : 0.0;
-      A[(size_t)i * n + j] = v;
-      if (row == j) dg[i] = v;
-    }
-  // the start: zero, the last solution, or the extrapolation of the last two
   const int h = *k.hist, warm = h < 2 ? h : 2;
   for (int t = tid; t < 3 * n; t += kChainThreads)
     p[t] = !warm ? 0.0 : (warm == 1 ? k.X[t] : X::sub(X::mul(2.0, k.X[t]), k.Xh[t]));
-  for (int t = tid; t < 3 * nl; t += kChainThreads) {
-    const int i = t % nl, c = t / nl, row = r0 + i;
+  // this thread's entry of the block's vectors (3 nl <= the block's threads)
+  const bool own = tid < 3 * nl;
+  const int oc = own ? tid / nl : 0, oi = own ? tid - oc * nl : 0, og = r0 + oi + oc * n;
+  if (own) {
     double U[3];
-    target_of(a, row, k.xyz, k.tgt, U[0], U[1], U[2]);
-    b[t] = X::div(X::sub(c == 0 ? U[0] : (c == 1 ? U[1] : U[2]), k.uvw[row + c * n]), a.dt);
+    target_of(a, r0 + oi, k.xyz, k.tgt, U[0], U[1], U[2]);
+    b[tid] = X::div(X::sub(oc == 0 ? U[0] : (oc == 1 ? U[1] : U[2]), k.uvw[og]), a.dt);
   }
   __syncthreads();
-  // v = A p on the block's rows
-  auto product = [&]() {
-    for (int i = wid; i < nl; i += nw) {
-      double s[3] = {0.0, 0.0, 0.0};
-      const double *Ai = A + (size_t)i * n;
-      for (int j = lane; j < n; j += 32) {
-        const double v = Ai[j];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) s[c] += v * p[j + c * n];
+  // the operator's rows
+  const int rw = (nl + NW - 1) / NW, i0 = wid * rw, ni = max(0, min(nl - i0, rw));  // rw <= RW
+  uint32_t chunks = 0;
+  for (int j0 = 0; j0 < n; j0 += 32) {
+    const int j = j0 + lane;
+    bool any = false;
+    for (int i = 0; i < ni; ++i) any = any || (j < n && may_couple_tab(a, tc, r0 + i0 + i, j));
+    if (!__any_sync(0xffffffffu, any)) continue;
+    chunks |= 1u << (j0 >> 5);
+    if (j < n)
+      for (int i = 0; i < ni; ++i) {
+        const int row = r0 + i0 + i;
+        const double v = may_couple_tab(a, tc, row, j) ? ivc_entry_tab(a, tw, tc, row, j, k.reg, ws) : 0.0;
+        A[(size_t)(i0 + i) * n + j] = v;
+        if (row == j) dg[i0 + i] = v;
       }
+  }
+  __syncthreads();
+  // ap = A p on the block's rows
+  auto product = [&]() {
+    double s[RW][3];
+#pragma unroll
+    for (int i = 0; i < RW; ++i) s[i][0] = s[i][1] = s[i][2] = 0.0;
+    for (uint32_t m = chunks; m; m &= m - 1) {
+      const int j = 32 * (__ffs(m) - 1) + lane;
+      if (j >= n) continue;
+      const double q0 = p[j], q1 = p[j + n], q2 = p[j + 2 * n];
+#pragma unroll
+      for (int i = 0; i < RW; ++i)
+        if (i < ni) {
+          const double v = A[(size_t)(i0 + i) * n + j];
+          s[i][0] += v * q0;
+          s[i][1] += v * q1;
+          s[i][2] += v * q2;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < RW; ++i) {
+      if (i >= ni) continue;  // (the same for the whole warp)
+#pragma unroll
       for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) s[c] += __shfl_xor_sync(0xffffffffu, s[c], o);
-      if (lane < 3) ap[i + lane * nl] = lane == 0 ? s[0] : (lane == 1 ? s[1] : s[2]);
+        for (int c = 0; c < 3; ++c) s[i][c] += __shfl_xor_sync(0xffffffffu, s[i][c], o);
+      if (lane < 3) ap[i0 + i + lane * nl] = lane == 0 ? s[i][0] : (lane == 1 ? s[i][1] : s[i][2]);
     }
     __syncthreads();
   };
   int red = 0;  // selects the reduction slots
-  // six sums over the block's rows (component c: u[] . v[], then w[] . w[]),
-  // sent to every block with the block's rows of v (= z)
-  auto reduce = [&](const double *u, const double *v, const double *w) {
-    if (wid < 6) {
-      const int c = wid % 3;
-      const double *f = wid < 3 ? u : w, *g = wid < 3 ? v : w;
-      double s = 0.0;
-      for (int i = lane; i < nl; i += 32) s += f[i + c * nl] * g[i + c * nl];
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (lane < kChainCtas) cl.map_shared_rank(slot, lane)[(red * kChainCtas + rank) * 6 + wid] = s;
-    }
-    for (int t = tid; t < 3 * nl * kChainCtas; t += kChainThreads) {
-      const int to = t / (3 * nl), q = t % (3 * nl), i = q % nl, c = q / nl;
-      cl.map_shared_rank(z, to)[r0 + i + c * n] = v[i + c * nl];
-    }
+  // warp w < 6: the sum of f . g over the block's rows of component w % 3, sent
+  // to every block; after the cluster barrier tot holds all blocks' sums
+  auto send = [&](const double *f, const double *g) {
+    const int c = wid % 3;
+    double s = 0.0;
+    for (int i = lane; i < nl; i += 32) s += f[i + c * nl] * g[i + c * nl];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane < CTAS) cl.map_shared_rank(slot, lane)[(red * CTAS + rank) * 6 + wid] = s;
+  };
+  auto collect = [&](int count) {
     cl.sync();
-    if (tid < 6) {
+    if (tid < count) {
       double s = 0.0;
-      for (int q = 0; q < kChainCtas; ++q) s += slot[(red * kChainCtas + q) * 6 + tid];
+      for (int q = 0; q < CTAS; ++q) s += slot[(red * CTAS + q) * 6 + tid];
       tot[tid] = s;
     }
     __syncthreads();
     red ^= 1;
   };
-  // r = b - A x0, z = r / diag; ap holds z of the block's rows for the sums
-  for (int t = tid; t < 3 * nl; t += kChainThreads) x[t] = p[r0 + t % nl + (t / nl) * n];
+  // r = b - A x0, z = r / diag (kept in ap for the sums)
+  if (own) x[tid] = p[og];
   product();
-  for (int t = tid; t < 3 * nl; t += kChainThreads) {
-    r[t] = b[t] - ap[t];
-    ap[t] = r[t] / dg[t % nl];
-  }
+  double zz = 0.0;
+  auto precondition = [&](double rr) {
+    zz = rr / dg[oi];
+    r[tid] = rr;
+    ap[tid] = zz;
+    for (int q = 0; q < CTAS; ++q) cl.map_shared_rank(z, q)[og] = zz;
+  };
+  if (own) precondition(b[tid] - ap[tid]);
   __syncthreads();
-  reduce(r, ap, b);
+  if (wid < 3) send(r, ap);
+  else if (wid < 6) send(b, b);
+  collect(6);
   double rz[3], bn[3];
   for (int c = 0; c < 3; ++c) {
     rz[c] = tot[c];
@@ -250,32 +289,19 @@ __device__ __forceinline__ void chain_cg(cgrp::cluster_group &cl, const IBCase &
   int it = 0;
   for (; it < 500; ++it) {
     product();
-    // (p of the block's rows is contiguous within a component)
-    if (wid < 3) {
-      double s = 0.0;
-      for (int i = lane; i < nl; i += 32) s += p[r0 + i + wid * n] * ap[i + wid * nl];
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (lane < kChainCtas) cl.map_shared_rank(slot, lane)[(red * kChainCtas + rank) * 6 + wid] = s;
-    }
-    cl.sync();
-    if (tid < 3) {
-      double s = 0.0;
-      for (int q = 0; q < kChainCtas; ++q) s += slot[(red * kChainCtas + q) * 6 + tid];
-      tot[tid] = s;
+    if (own) b[tid] = p[og];  // (b is needed no longer: the block's rows of p)
+    __syncthreads();
+    if (wid < 3) send(b, ap);
+    collect(3);
+    if (own) {
+      const double t = tot[oc], al = (t != 0.0) ? (oc == 0 ? rz[0] : (oc == 1 ? rz[1] : rz[2])) / t : 0.0;
+      x[tid] += al * p[og];
+      precondition(r[tid] - al * ap[tid]);
     }
     __syncthreads();
-    red ^= 1;
-    double alpha[3];
-    for (int c = 0; c < 3; ++c) alpha[c] = (tot[c] != 0.0) ? rz[c] / tot[c] : 0.0;
-    for (int t = tid; t < 3 * nl; t += kChainThreads) {
-      const int i = t % nl, c = t / nl;
-      const double al = c == 0 ? alpha[0] : (c == 1 ? alpha[1] : alpha[2]);
-      x[t] += al * p[r0 + i + c * n];
-      r[t] -= al * ap[t];
-      ap[t] = r[t] / dg[i];
-    }
-    __syncthreads();
-    reduce(r, ap, r);
+    if (wid < 3) send(r, ap);
+    else if (wid < 6) send(r, r);
+    collect(6);
     bool ok = true;
     double beta[3];
     for (int c = 0; c < 3; ++c) {
@@ -288,10 +314,9 @@ __device__ __forceinline__ void chain_cg(cgrp::cluster_group &cl, const IBCase &
       ++it;
       break;
     }
-    for (int t = tid; t < 3 * n; t += kChainThreads) {
-      const int c = t / n;
-      p[t] = z[t] + (c == 0 ? beta[0] : (c == 1 ? beta[1] : beta[2])) * p[t];
-    }
+    for (int j = tid; j < n; j += kChainThreads)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) p[j + c * n] = z[j + c * n] + beta[c] * p[j + c * n];
     __syncthreads();
   }
   // every block has read X, Xh and hist before its first cluster barrier
@@ -300,11 +325,10 @@ __device__ __forceinline__ void chain_cg(cgrp::cluster_group &cl, const IBCase &
     if (!done) atomicOr(k.status, 4);
     *k.hist = (h + 1 < 2) ? h + 1 : 2;
   }
-  for (int t = tid; t < 3 * nl; t += kChainThreads) {
-    const int e = r0 + t % nl + (t / nl) * n;
-    if (warm) k.Xh[e] = k.X[e];
-    k.X[e] = x[t];
-    k.F[e] = x[t];
+  if (own) {
+    if (warm) k.Xh[og] = k.X[og];
+    k.X[og] = x[tid];
+    k.F[og] = x[tid];
   }
 }
 
@@ -346,7 +370,7 @@ __device__ __forceinline__ void chain_body(const StepArgs &sa, const IBCase &k, 
   cl.sync();
   // 2: marker forces
   if (k.mode == 2) {
-    chain_cg<L>(cl, k, a, sh);
+    chain_cg<kChainCtas>(cl, k, a, sh);
   } else if (k.mode == 1) {
     for (int t = tid; t < 3 * n; t += kChainThreads) sh[t] = k.rhs[t % n + (t / n) * k.ld];
     __syncthreads();
@@ -428,4 +452,60 @@ __global__ void __cluster_dims__(kChainCtas, 1, 1) __launch_bounds__(kChainThrea
     k_ib_chain(const __grid_constant__ ChainArgs c) {
   extern __shared__ __align__(16) double sh[];
   chain_body<L, S>(c.s, c.k, c.k.a.kc, c.k.a.ks, c.k.a.komega, sh);
+}
+
+// ---------------------------------------------------------------------------
+// The batch's stages on the same functions.
+// ---------------------------------------------------------------------------
+// kinematics and interpolation, a warp per marker, with rho and u formed at the
+// stencils' cells (a macro pass over every band cell of the batch and a marker
+// kernel before it took 26 of 382 us per step on 32 cases); the spread force is
+// zero on entry (k_b_export leaves it so)
+template <class L, int S>
+__global__ void __launch_bounds__(128) k_b_interp(const IBCase *cs, const StepArgs *args, const ItemRef *list,
+                                                  int64_t cnt, const int *steps, const int *limit) {
+  const int lane = threadIdx.x & 31;
+  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < cnt; w += nw) {
+    const ItemRef e = list[w];
+    if (!live(steps, limit, e.c)) continue;
+    const IBCase &k = cs[e.c];
+    const int m = e.u;
+    if (lane == 0) {
+      if (m == 0) {
+        k.fsum[0] = k.fsum[1] = k.fsum[2] = 0.0;
+        atomicAnd(k.status, 1);  // (other warps may be raising bit 1 already)
+      }
+      if (k.moving) {
+        int s = steps[e.c];
+        if (s >= k.kin_steps) {
+          if (m == 0) atomicOr(k.status, 16);  // ran past its kinematics table
+          s = k.kin_steps - 1;
+        }
+        markers_one(k.a, k.kin[4 * s + 1], k.kin[4 * s + 2], k.kin[4 * s], m, k.xyz, k.ref, k.tgt, k.uvw, k.F);
+      }
+    }
+    __syncwarp();
+    chain_interp<L, S, false>(args[e.c], k, k.a, m, lane);
+  }
+}
+
+// the moving bodies' operator build and CG, a cluster per body (count, scan and
+// fill of a CSR operator and a one-block CG on it took 101 us for the 16
+// bodies of a 32-case batch; this takes 60 us, and its one launch leaves the
+// stored-inverse solves beside it undisturbed: 382 -> 333 us per batch step with
+// the interpolation above)
+constexpr int kBatchCgCtas = 8;
+__global__ void __cluster_dims__(kBatchCgCtas, 1, 1) __launch_bounds__(kChainThreads, 1)
+    k_b_cluster_cg(const IBCase *cs, const int *list, const int *steps, const int *limit) {
+  extern __shared__ __align__(16) double sh[];
+  __shared__ IBCase k;  // (not through the global table: its fields are read all through the solve)
+  const int c = list[blockIdx.x / kBatchCgCtas];
+  if (!live(steps, limit, c)) return;  // the same for the whole cluster
+  cgrp::cluster_group cl = cgrp::this_cluster();
+  for (int w = threadIdx.x; w < (int)(sizeof(IBCase) / sizeof(int)); w += blockDim.x)
+    reinterpret_cast<int *>(&k)[w] = reinterpret_cast<const int *>(cs + c)[w];
+  __syncthreads();
+  chain_cg<kBatchCgCtas>(cl, k, k.a, sh);
+  cl.sync();  // no block leaves while another may still write to it
 }

@@ -155,25 +155,6 @@ __global__ void __launch_bounds__(256) k_band_macro_list(StepArgs a, int blo0, i
     band_macro_cell<L, S>(a, blo0, blo1, blo2, bn0, bn1, nb, cells[r], EV, RHO);
 }
 
-// one block of kItemTile threads per band tile (case, first cell)
-template <class L, int S>
-__global__ void __launch_bounds__(kItemTile) k_band_macro_batch(const StepArgs *args,
-                                                                const BandDesc *bands,
-                                                                const ItemRef *tiles, int ntiles,
-                                                                const int *steps, const int *limit) {
-  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const ItemRef e = tiles[t];
-    const int c = e.c;
-    if (steps[c] >= limit[c]) continue;
-    const BandDesc &b = bands[c];
-    const int64_t u = (int64_t)e.u + threadIdx.x;
-    if (u >= b.nb) continue;
-    band_macro_cell<L, S>(args[c], b.blo[0], b.blo[1], b.blo[2], b.bn[0], b.bn[1], b.nb, u, b.EV,
-                          b.RHO);
-    if (b.EFI) b.EFI[u] = b.EFI[u + b.nb] = b.EFI[u + 2 * b.nb] = 0.0;  // spread target of this step
-  }
-}
-
 // Band macro of a level held in several boxes (caller-filled ghosts), the
 // EulerVel of IBMarkerDF::update_forcing (Source/IBM/IBMarkerDF.cpp:1541-1566)
 // followed by its FillBoundary (:702-703): a band cell takes rho, u from the
@@ -656,26 +637,6 @@ int batch_step_launch(ilbm_ctx *ctx, const StepArgs *d_args, const StepTile *d_t
   if (ntiles <= 0) return ILBM_OK;
   return ILBM_DISPATCH(ctx, launch_step_batch, ctx, d_args, d_tiles, ntiles, V, w, blocks, steps, limit,
                        st);
-}
-
-template <class L, int S>
-static int launch_band_macro_batch(ilbm_ctx *ctx, const StepArgs *d_args, const BandDesc *d_bands,
-                                   const ItemRef *d_tiles, int ntiles, const int *steps,
-                                   const int *limit, cudaStream_t st) {
-  const int blocks = std::min(ntiles, 4096);
-  k_band_macro_batch<L, S><<<blocks, kItemTile, 0, st>>>(d_args, d_bands, d_tiles, ntiles, steps, limit);
-  ctx->launches++;
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return cuda_fail(e, "batched band macro launch");
-  return ILBM_OK;
-}
-
-int batch_band_macro_launch(ilbm_ctx *ctx, const StepArgs *d_args, const BandDesc *d_bands,
-                            const ItemRef *d_tiles, int ntiles, const int *steps, const int *limit,
-                            cudaStream_t st) {
-  if (ntiles <= 0) return ILBM_OK;
-  return ILBM_DISPATCH(ctx, launch_band_macro_batch, ctx, d_args, d_bands, d_tiles, ntiles, steps,
-                       limit, st);
 }
 
 // resident blocks of w threads per SM for the batched level step

@@ -117,15 +117,6 @@ struct StepTile {
   uint32_t first, ghosts;
 };
 
-// Support band of an immersed body on a case's level (EV: 3 velocity
-// components, RHO: density, EFI: 3 spread-force components, zeroed by the
-// batched band macro when set; all band-sized).
-struct BandDesc {
-  int blo[3], bn[3];
-  int64_t nb;
-  double *EV, *RHO, *EFI;
-};
-
 // Work lists of the batched immersed-body stages: one entry per marker
 // (case, marker) and tiles of kItemTile band cells of one case (case, first
 // cell), so an item finds its case with one load.
