@@ -6,7 +6,7 @@
 // concatenated markers / band cells of every case (ib.cu), and the fused
 // collide-stream of every cell of every case is one persistent kernel that
 // walks a tile table of row segments and ghost-push chunks (k_step_batch,
-// lbm_step.cu).  Two consecutive steps (the two population buffers swap
+// level_step.cuh).  Two consecutive steps (the two population buffers swap
 // roles) are captured once as a CUDA graph and replayed.  The tile width and
 // the number of resident blocks come from ilbm_batch_tune, which times the
 // candidates on the batch itself.

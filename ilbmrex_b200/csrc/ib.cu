@@ -1240,11 +1240,6 @@ __device__ __forceinline__ void dense_row(const IBArgs &a, const double *rhs, co
   }
 }
 
-__global__ void __launch_bounds__(kDenseThreads) k_ivc_dense(IBArgs a, const double *rhs,
-                                                             const double *Ainv, int ld, double *F) {
-  dense_row(a, rhs, Ainv, ld, F, blockIdx.x);
-}
-
 // The same solve with A^-1 held in FP32 (the storage forms that keep their
 // populations in 4 or 2 bytes): half the bytes per step, products and sums
 // still in FP64; the rounding of A^-1 (2^-24 relative) is far below the
@@ -1286,11 +1281,6 @@ __device__ __forceinline__ void dense_row32(const IBArgs &a, const double *rhs, 
     for (int w = 0; w < kDenseThreads / 32; ++w) t += red[w][threadIdx.x];
     F[row + threadIdx.x * n] = X::add(F[row + threadIdx.x * n], t);
   }
-}
-
-__global__ void __launch_bounds__(kDenseThreads) k_ivc_dense32(IBArgs a, const double *rhs,
-                                                               const float *Ainv, int ld, double *F) {
-  dense_row32(a, rhs, Ainv, ld, F, blockIdx.x);
 }
 
 // kDenseRows rows per block: every thread has the loads of all its rows in
@@ -2011,7 +2001,7 @@ struct ilbm_ib {
   // last, d_Xh the one before it; the solves themselves advance it
   int *d_hist = nullptr;
   double *d_Xh = nullptr;
-  // fixed operator solved through its stored inverse (k_ivc_dense)
+  // fixed operator solved through its stored inverse (k_ivc_dense_rows)
   int ivc_solver = ILBM_IVC_AUTO;
   bool dense = false, dense_ready = false;
   int ld = 0;

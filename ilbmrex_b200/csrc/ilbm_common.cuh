@@ -210,8 +210,7 @@ struct Store<ILBM_STORAGE_F16_SCALED> {
   __device__ static __forceinline__ R load(const T *p, float s) { return __half2float(*p) * s; }
   __device__ static __forceinline__ R cvt(T v, float s) { return __half2float(v) * s; }
   __device__ static __forceinline__ void store(T *p, R v, float s) { *p = __float2half_rn(v / s); }
-  // si: the inverse factor scale / w_q
-  __device__ static __forceinline__ T pack(R v, float si) { return __float2half_rn(v * si); }
+  __device__ static __forceinline__ T pack(R v, float s) { return __float2half_rn(v / s); }
 };
 
 // rho, u of a cell from its populations and the previous force
@@ -505,11 +504,6 @@ __device__ __forceinline__ float post32(int q, float g, const Col32 &c) {
 struct Box3 {
   int lo[3], hi[3];
 };
-
-__host__ __device__ __forceinline__ bool in_box(const int *lo, const int *hi, int i, int j,
-                                                int k) {
-  return i >= lo[0] && i <= hi[0] && j >= lo[1] && j <= hi[1] && k >= lo[2] && k <= hi[2];
-}
 
 void set_error(const std::string &msg);
 int cuda_fail(cudaError_t e, const char *what);

@@ -7,19 +7,20 @@
 // writes halfway bounce-back ghosts for user_1 faces, pull-streams into f_new
 // and recomputes rho, u with F^n/2.
 //
-// B200 form: one pass.  Each thread owns one cell y, loads its Q populations
-// once (coalesced along i), recovers rho^n and u^n from them (bit-identical to
-// the stored macro because the reference computed it from the same f^n and
-// F^{n-1}; or reads macro_in), collides, and PUSHES f*(y,q) to f_out(y+c_q,q)
-// (wrapping periodic directions).  Populations whose pull source is a ghost
-// that nobody pushes from are completed by the thread that owns the
-// destination: bounce-back (f*(x,q_bar)), the pre-collision ghost value
+// B200 form: one pass, in level_step.cuh (this file holds the host side, the
+// macro, initialisation, derived-field and tagging kernels).  A cell's Q
+// populations are loaded once, rho^n and u^n recovered from them
+// (bit-identical to the stored macro because the reference computed it from
+// the same f^n and F^{n-1}; or read from macro_in), collided, and f*(y,q)
+// PUSHED to f_out(y+c_q,q) (wrapping periodic directions).  Populations whose
+// pull source is a ghost that nobody pushes from are completed by the owner of
+// the destination: bounce-back (f*(x,q_bar)), the pre-collision ghost value
 // (physical BC / coarse-fine), or, for a ghost covered by another box of the
-// level, that ghost collided in place.  Physical ghosts of layer 1 are
-// synthesised by a small prepass (self-fill mode) with the reference's
-// FillPatch rules, so the main kernel never evaluates boundary formulas.
-// Traffic per cell: Q loads + Q stores of the storage type (plus the force
-// band); no scratch copies.
+// level, that ghost collided in place.  What physical ghosts of layer 1 push
+// in (self-fill mode, the reference's FillPatch rules) comes from the ghost
+// blocks of the same launch, so the cells' code never evaluates boundary
+// formulas.  Traffic per cell: Q loads + Q stores of the storage type (plus
+// the force band); no scratch copies.
 #include <algorithm>
 #include <cstdlib>
 #include <cstdio>
@@ -41,8 +42,6 @@ int cuda_fail(cudaError_t e, const char *what) {
   set_error(std::string(what) + ": " + cudaGetErrorString(e));
   return ILBM_ERR_CUDA;
 }
-
-
 
 // ---------------------------------------------------------------------------
 // Macro pass (calculateMacroForcing) and equilibrium initialisation
@@ -326,7 +325,7 @@ static int fill_args(const ilbm_ctx *ctx, const ilbm_box &b, const ilbm_level_pa
   for (int q = 0; q < ctx->q; ++q) {
     const bool half = ctx->storage == ILBM_STORAGE_F16_SCALED;
     a.sf[q] = half ? float(ctx->w[q]) / scale16 : 1.0f;
-    a.si[q] = half ? float(double(scale16) / ctx->w[q]) : 1.0f;
+    a.si[q] = half ? float(1.0 / double(a.sf[q])) : 1.0f;
   }
   if (p) {
     for (int d = 0; d < 3; ++d) {

@@ -345,7 +345,7 @@ __device__ __forceinline__ void step_cell(const StepArgs &a, int i, int j, int k
   if (!edge) {
 #pragma unroll
     for (int q = 0; q < L::Q; ++q)
-      if (L::cx(q) == 0 ? own : (L::cx(q) > 0 ? ownp : ownm)) fob[a.doff[q]] = Store<S>::pack(f[q], a.si[q]);
+      if (L::cx(q) == 0 ? own : (L::cx(q) > 0 ? ownp : ownm)) fob[a.doff[q]] = Store<S>::pack(f[q], a.sf[q]);
     return;
   }
   const int st[3][2] = {{i == a.lo[0] ? a.face_lo[0] : 0, i == a.hi[0] ? a.face_hi[0] : 0},
@@ -368,9 +368,9 @@ __device__ __forceinline__ void step_cell(const StepArgs &a, int i, int j, int k
     const bool returned = c[0] != 0 && st[0][c[0] > 0] != 0;
     if (!((c[0] == 0 || returned) ? own : (c[0] > 0 ? ownp : ownm))) continue;
     if (link_reflects(m))
-      fob[a.loff[opposite<L>(q)]] = Store<S>::pack(f[q], a.si[opposite<L>(q)]);
+      fob[a.loff[opposite<L>(q)]] = Store<S>::pack(f[q], a.sf[opposite<L>(q)]);
     else if (link_arrives(m))
-      fob[a.doff[q] + wrap] = Store<S>::pack(f[q], a.si[q]);
+      fob[a.doff[q] + wrap] = Store<S>::pack(f[q], a.sf[q]);
   }
 }
 
@@ -404,7 +404,7 @@ __device__ __forceinline__ float2 f2(float x) { return make_float2(x, x); }
 // V consecutive populations, loaded and stored in one access and held in
 // registers as pairs in their storage form (4-byte: two floats, 2-byte: one
 // half2, converted when the pair is collided).  s / si: the direction's
-// storage factor and its inverse.
+// storage factor and its inverse, rounded to nearest.
 template <int B>
 struct Bytes;
 template <>
@@ -421,7 +421,7 @@ struct VecPair<ILBM_STORAGE_F32_SHIFT> {
   using Raw = float2;
   __device__ static __forceinline__ Raw zero() { return f2(0.0f); }
   __device__ static __forceinline__ float2 get(Raw r, float) { return r; }
-  __device__ static __forceinline__ Raw put(float2 v, float) { return v; }
+  __device__ static __forceinline__ Raw put(float2 v, float, float) { return v; }
   // the pair (b's second, c's first)
   __device__ static __forceinline__ Raw join(Raw b, Raw c) { return make_float2(b.y, c.x); }
   __device__ static __forceinline__ Raw from_up(Raw last) {  // the lane below's last cell, in second place
@@ -439,9 +439,22 @@ struct VecPair<ILBM_STORAGE_F16_SCALED> {
   __device__ static __forceinline__ float2 get(Raw r, float s) {
     return __fmul2_rn(__half22float2(*reinterpret_cast<const __half2 *>(&r)), f2(s));
   }
-  __device__ static __forceinline__ Raw put(float2 v, float si) {
-    const __half2 h = __float22half2_rn(__fmul2_rn(v, f2(si)));
+  // v / s rounded as the division rounds it: q = v * si, then one Markstein
+  // correction (exact for every 24-bit v with si the nearest 1 / s).  Both
+  // signs of zero come out as the division's; v is held to 1e20, which any
+  // scale that vec_width() lets through still takes to infinity, so that an infinite v
+  // does not meet itself in the remainder; NaN stays.
+  __device__ static __forceinline__ Raw put(float2 v, float s, float si) {
+    v = make_float2(held(v.x), held(v.y));
+    const float2 q = __fmul2_rn(v, f2(si));
+    const float2 r = __ffma2_rn(q, f2(s), make_float2(-v.x, -v.y));
+    const __half2 h = __float22half2_rn(__ffma2_rn(r, f2(-si), q));
     return *reinterpret_cast<const unsigned *>(&h);
+  }
+  __device__ static __forceinline__ float held(float v) {
+    float m;
+    asm("min.NaN.xorsign.abs.f32 %0, %1, %2;" : "=f"(m) : "f"(v), "f"(1e20f));
+    return m;
   }
   __device__ static __forceinline__ Raw join(Raw b, Raw c) { return __byte_perm(b, c, 0x5432); }
   __device__ static __forceinline__ Raw from_up(Raw last) { return __shfl_up_sync(0xffffffffu, last, 1); }
@@ -687,7 +700,7 @@ __device__ __forceinline__ void step_vector(const StepArgs &a, int x0, int j, in
     }
     collide_pair<L, MODE>(a, d, g);
 #pragma unroll
-    for (int q = 0; q < L::Q; ++q) f[q][h] = P::put(g[q], a.si[q]);
+    for (int q = 0; q < L::Q; ++q) f[q][h] = P::put(g[q], a.sf[q], a.si[q]);
   }
   // rows on a wrapping face deliver to the opposite row
   int64_t yw[2] = {0, 0}, zw[2] = {0, 0};
@@ -953,7 +966,10 @@ int vec_width(const StepArgs &a) {
   const uintptr_t out = (uintptr_t)(static_cast<const T *>(a.f_out) + off);
   const bool ok = in % (V * sizeof(T)) == 0 && out % (V * sizeof(T)) == 0 && a.fs0 % V == 0 &&
                   a.fs2 % V == 0 && (L::D == 2 || a.fs1 % V == 0);
-  return ok ? V : 1;
+  // F16: VecPair's division wants a scale within 2^-40 .. 2^40 (si is about
+  // two to three times it); any other takes the cell form, which divides
+  const bool scale_ok = S != ILBM_STORAGE_F16_SCALED || (a.si[0] > 0x1p-38f && a.si[0] < 0x1p40f);
+  return ok && scale_ok ? V : 1;
 }
 
 // the blocks of a planned launch; with ghost_blocks set, those of the ghost

@@ -281,7 +281,7 @@ int ilbm_advance_level(ilbm_ctx *ctx, const ilbm_box *box, const ilbm_level_para
                        ilbm_ib *ib, double dt, double time);
 /* sum over markers of F*dv from the last update_forcing (synchronises) */
 int ilbm_ib_last_marker_force_sum(ilbm_ib *ib, double out[3]);
-/* iterations of the last IVC conjugate-gradient solve (synchronises); the
+/* iterations of the last iterative IVC solve (synchronises); the
  * diagnostic counterpart of ibm.ivc_verbose (IBMarkerDF.cpp:1302-1313);
  * 0 when the system is solved through the stored inverse */
 int ilbm_ib_solver_stats(ilbm_ib *ib, int *cg_iterations);
@@ -594,8 +594,9 @@ int ilbm_batch_case_state(ilbm_batch *b, int case_id, int *parity, int64_t *step
  * force sum over the IB force region (3) and marker force sum (3); with out
  * NULL, *nrec = number available.  Synchronises. */
 int ilbm_batch_records(ilbm_batch *b, int case_id, double *out, int max_rec, int *nrec);
-/* tile width (threads per block: 64, 128, 256) and resident blocks per SM
- * (0: as many as fit) of the batched collide-stream */
+/* tile width (threads per block: 64, 128, 256; a thread of an aligned level's
+ * tile steps several cells) and resident blocks per SM (0: as many as fit) of
+ * the batched collide-stream */
 int ilbm_batch_set_tiles(ilbm_batch *b, int tile_w, int ctas_per_sm);
 /* times every tile width and block count on the batch itself (advancing every
  * case by the trial steps of each candidate) and keeps the fastest */
