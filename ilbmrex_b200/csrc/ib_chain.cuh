@@ -165,6 +165,10 @@ __device__ __forceinline__ void chain_dense_row(const IBCase &k, const TA *Ainv,
 // product of 48 rows.  Every block holds z and p of all markers; a block's z
 // rows and partial sums go to all blocks through distributed shared memory, and
 // each sums the partials in the same order, so all blocks take the same branches.
+// The first writes into other blocks' shared memory (z, slot) follow the
+// operator's build and need every block of the cluster to have started: the
+// function arrives at the cluster's barrier before that build and waits after
+// it, whatever its caller did before.
 template <int CTAS>
 __device__ __forceinline__ void chain_cg(cgrp::cluster_group &cl, const IBCase &k, const IBArgs &a, double *sh) {
   constexpr int NW = kChainThreads / 32, RW = 4;
@@ -176,6 +180,7 @@ __device__ __forceinline__ void chain_cg(cgrp::cluster_group &cl, const IBCase &
   double *x = p + 3 * n, *r = x + 3 * rows, *ap = r + 3 * rows, *b = ap + 3 * rows, *dg = b + 3 * rows;
   double *slot = dg + rows;  // [2][CTAS][6]
   double *tot = slot + 2 * CTAS * 6;
+  cl.barrier_arrive();  // (waited for before the first remote write)
   // the step's weight table, and the start: zero, the last solution, or the
   // extrapolation of the last two
 #pragma unroll 4
@@ -213,6 +218,7 @@ __device__ __forceinline__ void chain_cg(cgrp::cluster_group &cl, const IBCase &
         if (row == j) dg[i0 + i] = v;
       }
   }
+  cl.barrier_wait();  // every block of the cluster runs
   __syncthreads();
   // ap = A p on the block's rows
   auto product = [&]() {
