@@ -1039,7 +1039,8 @@ __device__ __forceinline__ void cheb_grid_body(cgrp::grid_group &grid, const IBA
                                                const double *tgt, const double *uvw, const int *rowptr,
                                                const int *col, const double *val, double lo, double hi,
                                                double *X_, double *Xh, double *work, double *F, double *partial,
-                                               double tol, int *hist, int *iters, double (*sh)[8], double *red) {
+                                               double tol, int *hist, int *status, int *iters, double (*sh)[8],
+                                               double *red) {
   const int n = a.n;
   const int h = *hist, warm = h < 2 ? h : 2;
   double *xa = work, *xb = work + 4 * (size_t)n, *D = work + 8 * (size_t)n, *B = work + 11 * (size_t)n;
@@ -1080,16 +1081,27 @@ __device__ __forceinline__ void cheb_grid_body(cgrp::grid_group &grid, const IBA
   block_partials(acc, 6, sh, partial);
   grid.sync();
   reduce_partials(partial, gridDim.x, 6, red);
-  // iterations: T_k(s1) >= |r0| / (tol |b|) for every component
+  // iterations: T_k(s1) >= |r0| / (tol |b|) for every component, 64 at most (T_64
+  // is 5e47 at the widest spectrum; a component with b = 0 takes them all).  A
+  // system without finite numbers, or further off than that, has not converged.
   double need = 1.0;
-  for (int c = 0; c < 3; ++c)
-    if (red[c] > 0.0) need = fmax(need, sqrt(red[c]) / (tol * sqrt(red[3 + c])));
+  bool ok = true, null = false;
+  for (int c = 0; c < 3; ++c) {
+    ok = ok && isfinite(red[c]) && isfinite(red[3 + c]);
+    if (!(red[c] > 0.0)) continue;
+    if (red[3 + c] > 0.0)
+      need = fmax(need, sqrt(red[c]) / (tol * sqrt(red[3 + c])));
+    else
+      null = true;
+  }
   int k = 1;
-  for (double t0 = 1.0, t1 = s1; t1 < need && k < 64; ++k) {
+  double t1 = s1;
+  for (double t0 = 1.0; ok && (null || t1 < need) && k < 64; ++k) {
     const double t2 = 2.0 * s1 * t1 - t0;
     t0 = t1;
     t1 = t2;
   }
+  ok = ok && t1 >= need;
   double rho = 1.0 / s1;
   double *x = xb, *y = xa;
   for (int it = 1; it < k; ++it) {
@@ -1113,6 +1125,7 @@ __device__ __forceinline__ void cheb_grid_body(cgrp::grid_group &grid, const IBA
   }
   if (gtid == 0) {
     *iters = k;
+    if (!ok) atomicOr(status, 4);
     *hist = (h + 1 < 2) ? h + 1 : 2;
   }
   for (int row = gh; row < n; row += nh)
@@ -1137,7 +1150,7 @@ __global__ void __launch_bounds__(256, 4) k_ivc_cg_grid(IBArgs a, const double *
   const double hi = *rowmax * (1.0 + 1.0e-12);  // (the same for every block: a uniform branch)
   if (reg > 0.0 && a.dv > 0.0 && hi <= kChebMax * reg) {
     cheb_grid_body(grid, a, xyz, tgt, uvw, rowptr, col, val, reg, hi, X_, Xh, work, F, partial, tol, hist,
-                   iters, sh, red);
+                   status, iters, sh, red);
     return;
   }
   cg_grid_body(grid, a, xyz, tgt, uvw, rowptr, col, val, diag, X_, Xh, work, F, partial, maxit, tol,
