@@ -1148,7 +1148,8 @@ __global__ void __launch_bounds__(256, 4) k_ivc_cg_grid(IBArgs a, const double *
   __shared__ double sh[8][8];
   __shared__ double red[8];
   const double hi = *rowmax * (1.0 + 1.0e-12);  // (the same for every block: a uniform branch)
-  if (reg > 0.0 && a.dv > 0.0 && hi <= kChebMax * reg) {
+  // (below reg: no operator, its build exceeded the capacity; the CG reports it)
+  if (reg > 0.0 && a.dv > 0.0 && hi >= reg && hi <= kChebMax * reg) {
     cheb_grid_body(grid, a, xyz, tgt, uvw, rowptr, col, val, reg, hi, X_, Xh, work, F, partial, tol, hist,
                    status, iters, sh, red);
     return;

@@ -1,7 +1,8 @@
 """The grid-wide IVC solve (more than 1024 markers): the Chebyshev iteration where
 the operator's largest row sum is at most twice its regularisation, CG above.
 Both against the stored inverse (FP64: relative L2 <= 1e-12 in populations, 1e-11
-in the force), and both report a flow that is no longer finite."""
+in the force), and both report what they cannot solve: a flow that is no longer
+finite, an operator that exceeded its capacity, on every step."""
 import numpy as np
 import pytest
 
@@ -73,6 +74,18 @@ def test_flow_that_is_not_finite_is_reported(reg, storage):
     s.step(2, record_force=True)
     s.f[0, 0, 180:200, 20:40] = float("nan")  # (the body's left edge is at x = 25)
     torch.cuda.synchronize()
+    for _ in range(2):
+        with pytest.raises(capi.IlbmError, match="did not converge"):
+            s.step(1, record_force=True)
+    s.close()
+
+
+def test_operator_beyond_its_capacity_is_reported_every_step():
+    """1,500 markers on 63 cells of circumference: about 200 neighbours per row
+    where the operator holds 96."""
+    s = solver(1.3, capi.IVC_CG, n=1500, D=20.0)
+    with pytest.raises(capi.IlbmError, match="capacity"):
+        s.step(1, record_force=True)
     for _ in range(2):
         with pytest.raises(capi.IlbmError, match="did not converge"):
             s.step(1, record_force=True)
