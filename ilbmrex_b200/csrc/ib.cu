@@ -3305,6 +3305,7 @@ __global__ void __launch_bounds__(kRecThreads) k_b_record(const IBCase *cs, int 
   }
   __syncthreads();
   if (threadIdx.x == 0) {
+    if (k.a.n > 0 && (k.status[0] & kLeftBand)) k.status[0] = (k.status[0] & ~kLeftBand) | 1;
     const int st = steps[c];
     double *r = k.rec + (size_t)(st % rec_slots) * 8;
     r[0] = fe[0];

@@ -47,10 +47,11 @@ __host__ __device__ inline size_t chain_shared(int mode, int n, int dim, int cta
 }
 
 // interpolation of marker m by one warp (interp_one / interp_seq with the
-// velocities formed at the stencil's cells); ORDERED: the reference's order
+// velocities formed at the stencil's cells); ORDERED: the reference's order;
+// left: the status bit of a stencil that leaves the band
 template <class L, int S, bool ORDERED>
 __device__ __forceinline__ void chain_interp(const StepArgs &sa, const IBCase &k, const IBArgs &a, int m,
-                                             int lane) {
+                                             int lane, int left) {
   const double px = k.xyz[m], py = k.xyz[m + a.n], pz = k.xyz[m + 2 * a.n];
   const double d = (a.dim == 3) ? X::mul(X::mul(a.dx[0], a.dx[1]), a.dx[2]) : X::mul(a.dx[0], a.dx[1]);
   int i0, j0, k0;
@@ -91,7 +92,7 @@ __device__ __forceinline__ void chain_interp(const StepArgs &sa, const IBCase &k
     }
     if (t < npts && dvl != 0.0 && ip >= ilo && ip <= ihi && jp >= jlo && jp <= jhi && kp >= klo && kp <= khi) {
       if (!in_band(a, ip, jp, kp)) {
-        atomicOr(k.status, 1);
+        atomicOr(k.status, left);
       } else {
         double m4[4];
         band_macro_value<L, S>(sa, ip, jp, kp, m4);
@@ -371,7 +372,7 @@ __device__ __forceinline__ void chain_body(const StepArgs &sa, const IBCase &k, 
   for (int m = gw; m < n; m += nw) {
     if (lane == 0 && k.moving) markers_one(a, kc, ks, om, m, k.xyz, k.ref, k.tgt, k.uvw, k.F);
     __syncwarp();
-    chain_interp<L, S, ORDERED>(sa, k, a, m, lane);
+    chain_interp<L, S, ORDERED>(sa, k, a, m, lane, 1);
   }
   cl.sync();
   // 2: marker forces
@@ -466,7 +467,10 @@ __global__ void __cluster_dims__(kChainCtas, 1, 1) __launch_bounds__(kChainThrea
 // kinematics and interpolation, a warp per marker, with rho and u formed at the
 // stencils' cells (a macro pass over every band cell of the batch and a marker
 // kernel before it took 26 of 382 us per step on 32 cases); the spread force is
-// zero on entry (k_b_export leaves it so)
+// zero on entry (k_b_export leaves it so).  The step's status starts here, in the
+// launch that may already raise its first bit: a stencil outside the band
+// raises kLeftBand, which k_b_record turns into status bit 1 at the step's end.
+constexpr int kLeftBand = 32;
 template <class L, int S>
 __global__ void __launch_bounds__(128) k_b_interp(const IBCase *cs, const StepArgs *args, const ItemRef *list,
                                                   int64_t cnt, const int *steps, const int *limit) {
@@ -480,7 +484,7 @@ __global__ void __launch_bounds__(128) k_b_interp(const IBCase *cs, const StepAr
     if (lane == 0) {
       if (m == 0) {
         k.fsum[0] = k.fsum[1] = k.fsum[2] = 0.0;
-        atomicAnd(k.status, 1);  // (other warps may be raising bit 1 already)
+        atomicAnd(k.status, kLeftBand);  // (other warps may be raising this step's already)
       }
       if (k.moving) {
         int s = steps[e.c];
@@ -492,7 +496,7 @@ __global__ void __launch_bounds__(128) k_b_interp(const IBCase *cs, const StepAr
       }
     }
     __syncwarp();
-    chain_interp<L, S, false>(args[e.c], k, k.a, m, lane);
+    chain_interp<L, S, false>(args[e.c], k, k.a, m, lane, kLeftBand);
   }
 }
 

@@ -7,7 +7,7 @@ warps' shares, and on both sides of the shared-memory limit (400 markers in 2D).
 import numpy as np
 import pytest
 
-from ilbmrex_b200 import cases
+from ilbmrex_b200 import capi, cases
 from ilbmrex_b200.lattice import D2Q9
 
 pytestmark = pytest.mark.gpu
@@ -46,4 +46,36 @@ def test_rebuilt_bodies_match_alone(counts):
         assert rel_l2(s.get_f(), ref.get_f()) <= 1e-12, n
         np.testing.assert_allclose(s.rec[3:5], ref.rec[3:5], rtol=1e-9, atol=1e-12, err_msg=str(n))
         ref.close()
+    B.close()
+
+
+def test_status_is_the_last_steps(tmp_path):
+    """A stencil that left its band on an earlier step (the body took another
+    one's checkpoint, and its own again) is no error of the batch's later steps;
+    one that leaves in the batch's last step is."""
+    def make(x, make_solver):
+        case, ib, init = cases.cylinder(nx=128, ny=64, D=16, center=(x, 31.7), U=0.05, Re=40, n_marker=48)
+        return make_solver(case, ib, init)
+
+    B = Batch(D2Q9, "f32")
+    s, other = make(32.3, B.solver), make(90.3, B.solver)
+    for t, name in ((s, "own"), (other, "other")):
+        t.step(2, record_force=True)
+        t.save_checkpoint(tmp_path / name)
+    s.load_checkpoint(tmp_path / "other")
+    with pytest.raises(capi.IlbmError, match="band"):
+        s.step(1, record_force=True)
+    s.load_checkpoint(tmp_path / "own")
+    s.ib_ready = True  # (its operator is built)
+    cid = B.add(s, max_steps=16)
+    B.step(3)
+    assert B.sync(cid).istep == 5
+    B.remove(cid)
+    s.load_checkpoint(tmp_path / "other")
+    s.ib_ready = True
+    B.add(s, max_steps=16)
+    with pytest.raises(capi.IlbmError, match="band"):
+        B.step(2)
+        B.progress()
+    other.close()
     B.close()
