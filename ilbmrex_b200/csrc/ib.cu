@@ -26,6 +26,7 @@
 #include <cooperative_groups.h>
 
 #include "batch_internal.h"
+#include "cluster_fit.h"
 #include "ilbm_common.cuh"
 #include "state_internal.h"
 #include "step_device.cuh"
@@ -2016,6 +2017,7 @@ struct ilbm_ib {
   int *d_hist = nullptr;
   double *d_Xh = nullptr;
   // fixed operator solved through its stored inverse (k_ivc_dense_rows)
+  bool chain = false;  // small enough for the one-launch chain, on a device that can run it
   int ivc_solver = ILBM_IVC_AUTO;
   bool dense = false, dense_ready = false;
   int ld = 0;
@@ -2389,7 +2391,8 @@ int enable_dense(ilbm_ib *ib) {
 
 }  // namespace
 
-static int chain_prepare(ilbm_ctx *ctx);
+static int chain_fits(ilbm_ctx *ctx, size_t shared, bool *fits);
+static size_t chain_shared_most(int coupling, int n, int dim);
 
 extern "C" {
 
@@ -2491,11 +2494,12 @@ int ilbm_ib_create(ilbm_ctx *ctx, const ilbm_ib_params *p, const ilbm_level_geom
       return rc;
     }
   }
-  if ((rc = chain_prepare(ctx))) {
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess && n <= kChainMaxMarkers && ib->nb <= kChainMaxBand &&
+      (rc = chain_fits(ctx, chain_shared_most(p->coupling_method, n, ib->dim), &ib->chain))) {
     ilbm_ib_destroy(ib);
     return rc;
   }
-  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     ilbm_ib_destroy(ib);
     return cuda_fail(e, "ilbm_ib_create");
@@ -2685,8 +2689,9 @@ static int ib_update(ilbm_ib *ib, const ilbm_box *boxes, int nbox, const ilbm_le
   // A small body takes its whole chain in one launch: a stored inverse once it
   // is built (the first step, below, builds it), a CG solve where the operator
   // is rebuilt every step anyway, or explicit coupling.  Larger bodies keep a
-  // launch per stage over the whole device.
-  if (!multi && single_ && ib->nb <= kChainMaxBand &&
+  // launch per stage over the whole device, and so do bodies on a device that
+  // cannot hold the chain's cluster.
+  if (ib->chain && !multi && single_ &&
       ib->n <= (ivc_ && !use_dense_ ? kChainMaxCg : kChainMaxMarkers) &&
       (!ivc_ || (use_dense_ ? ib->dense_ready : (ib->moving || ib->p.ivc_rebuild_matrix > 0)))) {
     int rc = launch_chain(ib, *box, lp, make_args(ib, dt, time), !ivc_ ? 0 : (use_dense_ ? 1 : 2), s);
@@ -3359,17 +3364,48 @@ static void chain_case(ilbm_ib *ib, const IBArgs &a, int mode, IBCase &k) {
   }
 }
 
-// what the chain kernel's launches need, once per body (on the body's device)
+// whether a cluster of `ctas` blocks of kernel k, kChainThreads threads and
+// `shared` bytes each (out of `most`, the largest launch's), can run on the
+// current device
+template <class K>
+static bool cluster_runs(K k, int ctas, size_t shared, size_t most) {
+  return cluster_fits(
+      [&]() -> int {
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+        if (e == cudaSuccess && ctas > 8)  // (beyond the portable size)
+          e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        return (int)e;
+      },
+      [&](int *resident) -> int {
+        cudaLaunchAttribute at = {};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = (unsigned)ctas;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cudaLaunchConfig_t c = {};
+        c.gridDim = dim3((unsigned)ctas);
+        c.blockDim = dim3(kChainThreads);
+        c.dynamicSmemBytes = shared;
+        c.attrs = &at;
+        c.numAttrs = 1;
+        return (int)cudaOccupancyMaxActiveClusters(resident, k, &c);
+      },
+      [] { cudaGetLastError(); });
+}
+
+// the chain kernel's attributes, and whether it can run with `shared` bytes per
+// block, once per body (on the body's device)
 template <class L, int S>
-static int chain_prepare_of(ilbm_ctx *) {
-  cudaError_t e = cudaFuncSetAttribute(k_ib_chain<L, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)chain_shared(2, kChainMaxCg, 3));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_ib_chain<L, S>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-  if (e != cudaSuccess) return cuda_fail(e, "body forcing: shared memory");
+static int chain_fits_of(size_t shared, bool *fits) {
+  *fits = cluster_runs(k_ib_chain<L, S>, kChainCtas, shared, chain_shared(2, kChainMaxCg, 3));
   return ILBM_OK;
 }
-static int chain_prepare(ilbm_ctx *ctx) { return ILBM_DISPATCH(ctx, chain_prepare_of, ctx); }
+static int chain_fits(ilbm_ctx *ctx, size_t shared, bool *fits) {
+  return ILBM_DISPATCH(ctx, chain_fits_of, shared, fits);
+}
+// the most shared memory a body's chain may ask for
+static size_t chain_shared_most(int coupling, int n, int dim) {
+  return coupling != 1 ? 0 : std::max(chain_shared(1, n, dim), n <= kChainMaxCg ? chain_shared(2, n, dim) : 0);
+}
 
 template <class L, int S>
 static int launch_chain_of(ilbm_ctx *ctx, const ChainArgs &c, cudaStream_t s) {
@@ -3466,13 +3502,12 @@ int ib_batch_create(ilbm_ctx *ctx, const std::vector<IBBatchCase> &cases, int re
   {
     cudaError_t e = cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_b_cluster_cg, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChainSharedMax);
     if (e != cudaSuccess) {
       ib_batch_destroy(b);
       return cuda_fail(e, "IB batch events");
     }
   }
+  const bool clusters = cluster_runs(k_b_cluster_cg, kBatchCgCtas, kChainSharedMax, kChainSharedMax);
   b->nc = (int)cases.size();
   b->rec_slots = std::max(1, rec_slots);
   std::vector<IBCase> hc(b->nc);
@@ -3558,7 +3593,8 @@ int ib_batch_create(ilbm_ctx *ctx, const std::vector<IBBatchCase> &cases, int re
     }
     moff[c + 1] = moff[c] + ib->n;
     boff[c + 1] = boff[c] + ib->nb;
-    const bool cluster = k.mode == 2 && k.rebuild && chain_shared(2, ib->n, ib->dim, kBatchCgCtas) <= kChainSharedMax;
+    const bool cluster =
+        clusters && k.mode == 2 && k.rebuild && chain_shared(2, ib->n, ib->dim, kBatchCgCtas) <= kChainSharedMax;
     for (int m = 0; m < ib->n; ++m) {
       mlist.push_back({c, m});
       if (k.rebuild && !cluster) rlist.push_back({c, m});

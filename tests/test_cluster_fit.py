@@ -1,0 +1,53 @@
+"""Bodies whose forcing takes a cluster launch keep working where the device
+refuses the cluster's attributes or cannot hold one: the decision (host code)
+against a fake runtime, and the launches a small body takes on this device."""
+import subprocess
+from pathlib import Path
+
+import pytest
+
+ROOT = Path(__file__).resolve().parents[1]
+
+PROGRAM = r"""
+#include "cluster_fit.h"
+#include <cstdio>
+int main() {
+  struct { int prepare, query, resident; } fake[] = {{0, 0, 3}, {0, 0, 1}, {0, 0, 0}, {1, 0, 3}, {0, 912, 3}};
+  for (auto &f : fake) {
+    int cleared = 0, asked = 0;
+    bool fits = ilbm::cluster_fits([&] { return f.prepare; },
+                                   [&](int *r) { ++asked; *r = f.resident; return f.query; }, [&] { ++cleared; });
+    std::printf("%d%d%d ", (int)fits, asked, cleared);
+  }
+}
+"""
+
+
+def test_refusals_are_no_error(tmp_path):
+    (tmp_path / "t.cpp").write_text(PROGRAM)
+    subprocess.run(["g++", "-std=c++17", f"-I{ROOT / 'ilbmrex_b200' / 'csrc'}", str(tmp_path / "t.cpp"), "-o",
+                    str(tmp_path / "t")], check=True)
+    out = subprocess.run([str(tmp_path / "t")], check=True, capture_output=True, text=True).stdout.split()
+    # (fits, query asked, error cleared)
+    assert out == ["110", "110", "010", "001", "011"]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,chain", [(64, True), (512, True), (513, False)])
+def test_small_bodies_take_the_cluster(n, chain):
+    """Explicit coupling: the chain, the cells outside the band and the band are
+    three launches; a launch per stage makes it six or more."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from ilbmrex_b200 import cases
+    from ilbmrex_b200.level import LevelSolver
+    case, ib, init = cases.cylinder(nx=96, ny=72, D=30, center=(40.3, 35.6), U=0.05, Re=40, n_marker=n, coupling=0)
+    s = LevelSolver(case, "f32", ib=ib)
+    s.set_macro(*init())
+    s.step(2)
+    before = s.ctx.launches()
+    s.step(1)
+    took = s.ctx.launches() - before
+    assert (took == 3) if chain else (took >= 6)
+    s.close()
