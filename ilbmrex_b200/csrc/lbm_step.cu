@@ -931,7 +931,9 @@ int level_step_impl(ilbm_ctx *ctx, const ilbm_box *boxes, int nbox, const ilbm_l
       return ILBM_ERR_ARG;
     }
   }
-  if (part == 0 && !mlo && (nbox > 1 || p->nlevel_boxes > 1)) return level_step_boxes(ctx, boxes, nbox, p);
+  // (the level's boxes are read in caller mode only)
+  if (part == 0 && !mlo && p->ghost_mode == ILBM_GHOST_CALLER && (nbox > 1 || p->nlevel_boxes > 1))
+    return level_step_boxes(ctx, boxes, nbox, p);
   for (int n = 0; n < nbox; ++n) {
     const ilbm_box &b = boxes[n];
     StepArgs a;
