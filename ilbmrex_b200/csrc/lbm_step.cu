@@ -789,18 +789,19 @@ __global__ void __launch_bounds__(256) k_tags(TagArgs g, const R *vor, unsigned 
 template <class L, int S>
 static int launch_boxes(ilbm_ctx *ctx, StepBoxes &p, const StepBoxes &whole) {
   if (!launch_step_boxes<L, S>(ctx, p, ctx->stream)) {
-    // a very large box: one launch per box, with the level's boxes beside it
+    // too many cells together: one launch per box (in slices along the last
+    // dimension where it alone is too large), with the level's boxes beside it
     for (int n = 0; n < whole.nbox; ++n) {
       StepBoxes one = whole;
       one.nbox = 1;
       one.a[0] = whole.a[n];
       const int e = L::D - 1, last = one.a[0].rhi[e];
-      int64_t slice = 1;
+      int64_t slice = 1;  // below 2^28: the offsets of a neighbouring layer fit 32 bits
       for (int d = 0; d < e; ++d) slice *= one.a[0].rhi[d] - one.a[0].rlo[d] + 1;
-      const int most = (int)std::max<int64_t>(1, (int64_t)(1 << 26) / slice);
-      for (int s = one.a[0].rlo[e]; s <= last; s += most) {
-        one.a[0].rlo[e] = s;
-        one.a[0].rhi[e] = std::min(last, s + most - 1);
+      const int64_t most = std::max<int64_t>(1, kMaxLaunchCells / slice);
+      for (int64_t s = one.a[0].rlo[e]; s <= last; s += most) {
+        one.a[0].rlo[e] = (int)s;
+        one.a[0].rhi[e] = (int)std::min<int64_t>(last, s + most - 1);
         if (!launch_step_boxes<L, S>(ctx, one, ctx->stream)) {
           set_error("box too large for one launch");
           return ILBM_ERR_RANGE;

@@ -1023,12 +1023,14 @@ template <class L, int S>
 bool launch_step_boxes(ilbm_ctx *ctx, StepBoxes &p, cudaStream_t st) {
   constexpr int VV = StepVec<L, S>::value;
   int V = VV;
+  int64_t total = 0;
   for (int n = 0; n < p.nbox; ++n) {
     V = std::min(V, vec_width<L, S>(p.a[n]));
     int64_t cells = 1;
     for (int d = 0; d < L::D; ++d) cells *= p.a[n].rhi[d] - p.a[n].rlo[d] + 1;
-    if (cells > (1 << 26)) return false;  // (2^30 vectors in all 16 boxes)
+    total += cells;
   }
+  if (total > kMaxLaunchCells) return false;
   uint32_t blocks = 0;
   for (int n = 0; n < p.nbox; ++n) {
     plan_vectors(p.a[n], L::D, V);

@@ -16,6 +16,10 @@ __host__ __device__ constexpr uint32_t step_vectors_per_block(int V, uint32_t n)
   return V > 1 ? n / 32u * kOwned : n;
 }
 
+// cells of one launch: its vectors are counted in 32 bits and divided as
+// numbers below 2^31 (fast_div), the halo lanes' and ghost blocks' included
+constexpr int64_t kMaxLaunchCells = 1 << 30;
+
 // magic of a division by d (1 <= d < 2^31) of numbers below 2^31 (fast_div)
 DivMagic div_magic(uint32_t d);
 // the cells [rlo, rhi] of a launch as a sequence of V-cell vectors; false: empty
@@ -31,7 +35,7 @@ template <class L, int S>
 void launch_cells(ilbm_ctx *ctx, const StepArgs &a, cudaStream_t st, bool with_ghosts, bool singly = false);
 
 // the boxes of a level (whole, with their ghost shells) in one launch; false,
-// with nothing launched: a box is too large for it
+// with nothing launched: they hold more than kMaxLaunchCells cells
 template <class L, int S>
 bool launch_step_boxes(ilbm_ctx *ctx, StepBoxes &p, cudaStream_t st);
 

@@ -33,3 +33,38 @@ def test_self_filled_level_ignores_the_level_boxes(count, table):
         out.append(s.get_f())
         s.close()
     np.testing.assert_array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("nx,ny", [((1 << 26) - 4, 1), ((1 << 26) + 5, 1), (32771, 32800)])
+def test_box_of_very_many_cells(nx, ny):
+    """One box of a level of two, its rows longer or its cells more (2^30 and
+    some) than one several-box launch takes: the same bits as the box taken as
+    its level's only one (no ghost cell is covered by the other box)."""
+    from ilbmrex_b200.level import alloc_populations
+    ctx = Context(D2Q9, "f16")
+    dev = torch.device("cuda")
+    fi = alloc_populations(9, 1, ny + 2, nx + 2, torch.float16, dev)
+    outs = [alloc_populations(9, 1, ny + 2, nx + 2, torch.float16, dev) for _ in range(2)]
+    torch.manual_seed(1)
+    for q in range(9):
+        fi[q].normal_(0.0, 20.0)
+    case = cases.LevelCase(D2Q9, (nx + 300, ny + 40, 1), nu=0.06)
+    for fo, boxes in zip(outs, (1, 2)):
+        b = capi.Box_t()
+        for d, (lo, hi) in enumerate(((100, 100 + nx - 1), (20, 20 + ny - 1), (0, 0))):
+            b.lo[d], b.hi[d] = lo, hi
+        b.ngrow_f, b.ngrow_m = 1, 2
+        fs = fi.stride()
+        b.fstride[:] = [fs[2], fs[1], fs[0]]
+        b.f_in, b.f_out = fi.data_ptr(), fo.data_ptr()
+        lb = (C.c_int * 12)(100, 20, 0, 100 + nx - 1, 20 + ny - 1, 0, 0, 0, 0, 9, 4, 0)
+        p = level_params(case, uniform_force=False)
+        p.ghost_mode, p.nlevel_boxes = capi.GHOST_CALLER, boxes
+        p.level_boxes = C.cast(lb, C.POINTER(C.c_int))
+        torch.cuda.synchronize()
+        capi.check(ctx.L.ilbm_level_step(ctx.h, C.byref(b), 1, C.byref(p)), "level_step")
+        ctx.sync()
+    for q in range(9):
+        assert torch.equal(outs[0][q, 0, 1:-1, 1:-1], outs[1][q, 0, 1:-1, 1:-1])
+    assert float(outs[0][1, 0, -2, 1:-1].abs().max()) > 0.0
+    ctx.close()
