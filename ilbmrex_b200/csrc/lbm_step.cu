@@ -620,10 +620,10 @@ int batch_plan(const ilbm_ctx *ctx, StepArgs *args, int n, int *V) {
   }
   for (int c = 0; c < n; ++c) {
     const StepArgs &a = args[c];
-    int64_t cells = 1;
-    for (int d = 0; d < ctx->dim; ++d) cells *= a.rhi[d] - a.rlo[d] + 1;
-    if (cells > (1 << 30)) {
-      set_error("batched case: 2^30 cells at most");
+    int64_t vectors = (a.rhi[0] - a.rlo[0] + *V) / *V;  // (a self-filled box: its rows start on vectors)
+    for (int d = 1; d < ctx->dim; ++d) vectors *= a.rhi[d] - a.rlo[d] + 1;
+    if (vectors >= INT32_MAX - 1024) {  // (fast_div, with the tiles' last lanes beyond the end)
+      set_error("batched case: fewer than 2^31 vectors of cells (a cell each in unaligned rows)");
       return ILBM_ERR_RANGE;
     }
     plan_vectors(args[c], ctx->dim, *V);

@@ -68,3 +68,37 @@ def test_box_of_very_many_cells(nx, ny):
         assert torch.equal(outs[0][q, 0, 1:-1, 1:-1], outs[1][q, 0, 1:-1, 1:-1])
     assert float(outs[0][1, 0, -2, 1:-1].abs().max()) > 0.0
     ctx.close()
+
+
+@pytest.mark.parametrize("nx,ny", [(1024, 96), (32771, 32800)])
+def test_batched_case_of_very_many_cells(nx, ny):
+    """One step of a batched periodic case, of more than 2^30 cells too, is the
+    level step's, bit for bit."""
+    from ilbmrex_b200.level import alloc_populations
+    ctx = Context(D2Q9, "f16")
+    dev = torch.device("cuda")
+    fi, one, two = (alloc_populations(9, 1, ny + 2, nx + 2, torch.float16, dev) for _ in range(3))
+    torch.manual_seed(2)
+    for q in range(9):
+        fi[q].normal_(0.0, 20.0)
+    case = cases.LevelCase(D2Q9, (nx, ny, 1), nu=0.06)
+    p = level_params(case, uniform_force=False)
+    b = capi.Box_t()
+    for d, n in enumerate((nx, ny, 1)):
+        b.lo[d], b.hi[d] = 0, n - 1
+    b.ngrow_f, b.ngrow_m = 1, 2
+    fs = fi.stride()
+    b.fstride[:] = [fs[2], fs[1], fs[0]]
+    b.f_in, b.f_out = fi.data_ptr(), one.data_ptr()
+    torch.cuda.synchronize()
+    capi.check(ctx.L.ilbm_level_step(ctx.h, C.byref(b), 1, C.byref(p)), "level_step")
+    h, cid = C.c_void_p(), C.c_int()
+    capi.check(ctx.L.ilbm_batch_create(ctx.h, 8, C.byref(h)), "batch_create")
+    b.f_out = two.data_ptr()
+    capi.check(ctx.L.ilbm_batch_add(h, C.byref(b), C.byref(p), None, 1.0, 0.0, 4, C.byref(cid)), "batch_add")
+    capi.check(ctx.L.ilbm_batch_step(h, 1), "batch_step")
+    ctx.sync()
+    for q in range(9):
+        assert torch.equal(one[q, 0, 1:-1, 1:-1], two[q, 0, 1:-1, 1:-1])
+    ctx.L.ilbm_batch_destroy(h)
+    ctx.close()
