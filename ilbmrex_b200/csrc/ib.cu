@@ -2691,7 +2691,11 @@ static int ib_update(ilbm_ib *ib, const ilbm_box *boxes, int nbox, const ilbm_le
   // is rebuilt every step anyway, or explicit coupling.  Larger bodies keep a
   // launch per stage over the whole device, and so do bodies on a device that
   // cannot hold the chain's cluster.
-  if (ib->chain && !multi && single_ &&
+  // The chain zeroes box->force while it still reads velocities, so a call whose
+  // force and force_prev are one array (F^{n-1} on entry, F^n on return) and that
+  // recovers them from it goes by stages, which write the force last.
+  const bool in_place = box->force == box->force_prev && !box->macro_in;
+  if (ib->chain && !multi && single_ && !in_place &&
       ib->n <= (ivc_ && !use_dense_ ? kChainMaxCg : kChainMaxMarkers) &&
       (!ivc_ || (use_dense_ ? ib->dense_ready : (ib->moving || ib->p.ivc_rebuild_matrix > 0)))) {
     int rc = launch_chain(ib, *box, lp, make_args(ib, dt, time), !ivc_ ? 0 : (use_dense_ ? 1 : 2), s);

@@ -1,0 +1,46 @@
+"""Calls of ilbm_ib_update_forcing at the edges of what it takes, for bodies
+whose chain is one launch and for those that take a launch per stage (FP64:
+the exported force bit for bit, explicit coupling summing in a fixed order)."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from ilbmrex_b200 import capi, cases
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():
+    pytest.skip("needs a CUDA device", allow_module_level=True)
+
+from ilbmrex_b200.level import LevelSolver  # noqa: E402
+
+
+def stepped(n, cy=35.6, coupling=0, steps=3):
+    case, ib, init = cases.cylinder(nx=96, ny=72, D=30, center=(40.3, cy), U=0.05, Re=40, n_marker=n,
+                                    coupling=coupling)
+    s = LevelSolver(case, "f64", ib=ib)
+    s.set_macro(*init())
+    s.step(steps)
+    s.ctx.sync()
+    return s
+
+
+def update(s, box):
+    torch.cuda.synchronize()
+    capi.check(s.L.ilbm_ib_update_forcing(s.ib, C.byref(box), 1, C.byref(s.params), s.case.dt, s.time), "update_forcing")
+    s.ctx.sync()
+
+
+@pytest.mark.parametrize("n", [60, 512, 513])
+def test_force_in_place(n):
+    """One array for F^{n-1} (read) and F^n (written)."""
+    s = stepped(n)
+    apart = torch.zeros_like(s.force_prev)
+    update(s, s._box(s.f, None, force=apart, force_prev=s.force_prev))
+    one = s.force_prev.clone()
+    update(s, s._box(s.f, None, force=one, force_prev=one))
+    assert float(apart.abs().max()) > 0.0
+    np.testing.assert_array_equal(one.cpu().numpy(), apart.cpu().numpy())
+    s.close()
