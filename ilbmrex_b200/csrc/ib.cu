@@ -2695,7 +2695,11 @@ static int ib_update(ilbm_ib *ib, const ilbm_box *boxes, int nbox, const ilbm_le
   // force and force_prev are one array (F^{n-1} on entry, F^n on return) and that
   // recovers them from it goes by stages, which write the force last.
   const bool in_place = box->force == box->force_prev && !box->macro_in;
-  if (ib->chain && !multi && single_ && !in_place &&
+  // Caller-filled macro fields whose band reaches over a periodic face: the
+  // stages replace the band's ghost velocities by their periodic images
+  // (FillBoundary, IBMarkerDF.cpp:702-703); the chain reads the ghosts as given.
+  const bool images = periodic_band && box->macro_in && lp->ghost_mode != ILBM_GHOST_SELF;
+  if (ib->chain && !multi && single_ && !in_place && !images &&
       ib->n <= (ivc_ && !use_dense_ ? kChainMaxCg : kChainMaxMarkers) &&
       (!ivc_ || (use_dense_ ? ib->dense_ready : (ib->moving || ib->p.ivc_rebuild_matrix > 0)))) {
     int rc = launch_chain(ib, *box, lp, make_args(ib, dt, time), !ivc_ ? 0 : (use_dense_ ? 1 : 2), s);

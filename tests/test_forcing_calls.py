@@ -44,3 +44,30 @@ def test_force_in_place(n):
     assert float(apart.abs().max()) > 0.0
     np.testing.assert_array_equal(one.cpu().numpy(), apart.cpu().numpy())
     s.close()
+
+
+@pytest.mark.parametrize("n", [40, 513])
+def test_caller_filled_band_over_a_periodic_face(n):
+    """Caller-filled macro fields: the band's ghosts beyond a periodic face are
+    their images whatever the caller's ghost cells hold there."""
+    s = stepped(n, cy=6.2)
+    m = torch.zeros_like(s.macro)
+    s._valid(m, s.gm).copy_(torch.as_tensor(s.get_macro()).to(m.device))
+    p = s.params
+    s.params = type(p).from_buffer_copy(p)
+    s.params.ghost_mode = capi.GHOST_CALLER
+    out = []
+    for fill in (False, True):
+        if fill:  # the two ghost rows on each y face
+            m[..., 0:2, :] = m[..., -4:-2, :]
+            m[..., -2:, :] = m[..., 2:4, :]
+        f = torch.zeros_like(s.force_prev)
+        update(s, s._box(s.f, None, macro_in=m, force=f))
+        out.append(f.cpu().numpy())
+    s.params = p
+    f = torch.zeros_like(s.force_prev)
+    update(s, s._box(s.f, None, force=f, force_prev=s.force_prev))  # self-filled, from the populations
+    assert np.abs(out[1]).max() > 0.0
+    np.testing.assert_array_equal(out[0], out[1])
+    np.testing.assert_array_equal(f.cpu().numpy(), out[1])
+    s.close()
