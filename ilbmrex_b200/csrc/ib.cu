@@ -3372,12 +3372,12 @@ static void chain_case(ilbm_ib *ib, const IBArgs &a, int mode, IBCase &k) {
   }
 }
 
-// whether a cluster of `ctas` blocks of kernel k, kChainThreads threads and
-// `shared` bytes each (out of `most`, the largest launch's), can run on the
-// current device
+// the clusters of `ctas` blocks of kernel k, kChainThreads threads and `shared`
+// bytes each (out of `most`, the largest launch's), that the current device
+// runs at once
 template <class K>
-static bool cluster_runs(K k, int ctas, size_t shared, size_t most) {
-  return cluster_fits(
+static int clusters_of(K k, int ctas, size_t shared, size_t most) {
+  return clusters_resident(
       [&]() -> int {
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
         if (e == cudaSuccess && ctas > 8)  // (beyond the portable size)
@@ -3404,7 +3404,7 @@ static bool cluster_runs(K k, int ctas, size_t shared, size_t most) {
 // block, once per body (on the body's device)
 template <class L, int S>
 static int chain_fits_of(size_t shared, bool *fits) {
-  *fits = cluster_runs(k_ib_chain<L, S>, kChainCtas, shared, chain_shared(2, kChainMaxCg, 3));
+  *fits = clusters_of(k_ib_chain<L, S>, kChainCtas, shared, chain_shared(2, kChainMaxCg, 3)) > 0;
   return ILBM_OK;
 }
 static int chain_fits(ilbm_ctx *ctx, size_t shared, bool *fits) {
@@ -3454,7 +3454,7 @@ struct IBBatch {
   ItemRef *d_mlist = nullptr, *d_rlist = nullptr, *d_dlist = nullptr, *d_btiles = nullptr;
   int *d_cgcase = nullptr;
   int ncg = 0;
-  // rebuilding bodies whose rows fit a cluster's shared memory (k_b_cluster_cg)
+  // bodies solved by a cluster each (k_b_cluster_cg)
   int *d_clcase = nullptr;
   int ncl = 0;
   size_t cl_shared = 0;
@@ -3502,6 +3502,17 @@ void ib_batch_destroy(IBBatch *b) {
   delete b;
 }
 
+// a batched body's solve (IBCase::mode), and whether its operator is rebuilt every step
+static int batch_mode(const ilbm_ib *ib) {
+  if (ib->p.coupling_method != 1) return 0;
+  const bool dense = ib->dense && ib->dense_ready && !ib->moving && ib->p.ivc_rebuild_matrix == 0 &&
+                     ib->ivc_solver != ILBM_IVC_CG;
+  return dense ? 1 : 2;
+}
+static bool batch_rebuilds(const ilbm_ib *ib) {
+  return batch_mode(ib) == 2 && (ib->moving || ib->p.ivc_rebuild_matrix > 0);
+}
+
 int ib_batch_create(ilbm_ctx *ctx, const std::vector<IBBatchCase> &cases, int rec_slots,
                     IBBatch **out) {
   *out = nullptr;
@@ -3515,7 +3526,26 @@ int ib_batch_create(ilbm_ctx *ctx, const std::vector<IBBatchCase> &cases, int re
       return cuda_fail(e, "IB batch events");
     }
   }
-  const bool clusters = cluster_runs(k_b_cluster_cg, kBatchCgCtas, kChainSharedMax, kChainSharedMax);
+  // The bodies' CG: a cluster each where every body solved by CG can have one
+  // (its operator rebuilt each step, its rows within the blocks' shared memory)
+  // and they run in two waves at most; else the sparse operators and a block
+  // each, in one set of launches for all.  Both kinds in a row, or a third wave,
+  // cost more than the clusters give.  Measured (B200, 15 clusters a wave, us per
+  // step with clusters / without): 15 bodies of 240 markers 56 / 77 FP32, 96 / 130
+  // FP64; 28 of them 102 / 111 and 178 / 172; 32 of 200 markers 125 / 111 and 223 / 172;
+  // 12 bodies of 200 and 420 markers by turns 106 / 91 and 196 / 158.
+  bool clusters = true;
+  int nclusters = 0;
+  for (const IBBatchCase &x : cases) {
+    const ilbm_ib *ib = x.ib;
+    if (!ib || batch_mode(ib) != 2) continue;
+    const size_t sh = chain_shared(2, ib->n, ib->dim, kBatchCgCtas);
+    clusters = clusters && batch_rebuilds(ib) && sh <= kChainSharedMax;
+    b->cl_shared = std::max(b->cl_shared, sh);
+    ++nclusters;
+  }
+  clusters = clusters && nclusters > 0 &&
+             nclusters <= 2 * clusters_of(k_b_cluster_cg, kBatchCgCtas, b->cl_shared, kChainSharedMax);
   b->nc = (int)cases.size();
   b->rec_slots = std::max(1, rec_slots);
   std::vector<IBCase> hc(b->nc);
@@ -3562,10 +3592,8 @@ int ib_batch_create(ilbm_ctx *ctx, const std::vector<IBBatchCase> &cases, int re
     k.moving = ib->moving ? 1 : 0;
     for (int d = 0; d < ib->dim; ++d)
       k.periodic_band = k.periodic_band || (ib->g.periodic[d] && ib->blo[d] < 0);
-    const bool dense = ivc && ib->dense && ib->dense_ready && !ib->moving &&
-                       ib->p.ivc_rebuild_matrix == 0 && ib->ivc_solver != ILBM_IVC_CG;
-    k.mode = !ivc ? 0 : (dense ? 1 : 2);
-    k.rebuild = (k.mode == 2 && (ib->moving || ib->p.ivc_rebuild_matrix > 0)) ? 1 : 0;
+    k.mode = batch_mode(ib);
+    k.rebuild = batch_rebuilds(ib) ? 1 : 0;
     k.rowptr = ib->d_rowptr;
     k.col = ib->d_col;
     k.val = ib->d_val;
@@ -3601,8 +3629,7 @@ int ib_batch_create(ilbm_ctx *ctx, const std::vector<IBBatchCase> &cases, int re
     }
     moff[c + 1] = moff[c] + ib->n;
     boff[c + 1] = boff[c] + ib->nb;
-    const bool cluster =
-        clusters && k.mode == 2 && k.rebuild && chain_shared(2, ib->n, ib->dim, kBatchCgCtas) <= kChainSharedMax;
+    const bool cluster = clusters && k.mode == 2;
     for (int m = 0; m < ib->n; ++m) {
       mlist.push_back({c, m});
       if (k.rebuild && !cluster) rlist.push_back({c, m});
@@ -3613,7 +3640,6 @@ int ib_batch_create(ilbm_ctx *ctx, const std::vector<IBBatchCase> &cases, int re
     k.ntile = (int)btiles.size() - k.tile0;
     if (cluster) {
       clcase.push_back(c);
-      b->cl_shared = std::max(b->cl_shared, chain_shared(2, ib->n, ib->dim, kBatchCgCtas));
     } else if (k.mode == 2) {
       cgcase.push_back(c);
     }

@@ -1,9 +1,11 @@
 """The batch's solve of bodies whose operator is rebuilt every step: a cluster of
-eight blocks per body where its rows fit the blocks' shared memory, the sparse
-operator and one block's CG above.  Each body in the batch equals the same body
-advanced alone (relative L2 <= 1e-12 in populations, records to 1e-9: both solve
-to 1e-14), at marker counts with blocks that own no rows, around the blocks' and
-warps' shares, and on both sides of the shared-memory limit (400 markers in 2D)."""
+eight blocks per body where the rows of all of them fit the blocks' shared
+memory and all clusters run in two waves, the sparse operators and one block's CG
+each otherwise.  Each body in the batch equals the same body advanced alone
+(relative L2 <= 1e-12 in populations, records to 1e-9: both solve to 1e-14), at
+marker counts with blocks that own no rows, around the blocks' and warps'
+shares, on both sides of the shared-memory limit (400 markers in 2D), with bodies
+of both sides, and with more bodies than one and two waves hold."""
 import numpy as np
 import pytest
 
@@ -31,7 +33,8 @@ def body(n):
 
 
 @pytest.mark.parametrize("counts", [(1, 2, 7, 8, 9), (15, 16, 17, 63, 65), (127, 128, 129, 241),
-                                    (399, 400, 401, 449)])
+                                    (399, 400), (401, 449), (33, 400, 401), (1, 9, 17, 33) * 6, (1, 9, 17, 33) * 10],
+                         ids=lambda c: "-".join(map(str, c[:4])) + f"x{len(c)}")
 def test_rebuilt_bodies_match_alone(counts):
     steps = 5
     B = Batch(D2Q9, "f64")

@@ -15,9 +15,9 @@ int main() {
   struct { int prepare, query, resident; } fake[] = {{0, 0, 3}, {0, 0, 1}, {0, 0, 0}, {1, 0, 3}, {0, 912, 3}};
   for (auto &f : fake) {
     int cleared = 0, asked = 0;
-    bool fits = ilbm::cluster_fits([&] { return f.prepare; },
-                                   [&](int *r) { ++asked; *r = f.resident; return f.query; }, [&] { ++cleared; });
-    std::printf("%d%d%d ", (int)fits, asked, cleared);
+    int n = ilbm::clusters_resident([&] { return f.prepare; },
+                                    [&](int *r) { ++asked; *r = f.resident; return f.query; }, [&] { ++cleared; });
+    std::printf("%d%d%d ", n, asked, cleared);
   }
 }
 """
@@ -28,8 +28,8 @@ def test_refusals_are_no_error(tmp_path):
     subprocess.run(["g++", "-std=c++17", f"-I{ROOT / 'ilbmrex_b200' / 'csrc'}", str(tmp_path / "t.cpp"), "-o",
                     str(tmp_path / "t")], check=True)
     out = subprocess.run([str(tmp_path / "t")], check=True, capture_output=True, text=True).stdout.split()
-    # (fits, query asked, error cleared)
-    assert out == ["110", "110", "010", "001", "011"]
+    # (clusters, query asked, error cleared)
+    assert out == ["310", "110", "010", "001", "011"]
 
 
 @pytest.mark.gpu
