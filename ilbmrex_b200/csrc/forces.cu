@@ -143,11 +143,13 @@ __global__ void k_final_sum(const double *partial, int nparts, double *out,
 }
 
 // The sum over a small region in one launch (k_force_partial and k_final_sum
-// are two, of which the second waits for the first: 10 us on the device for the
-// 2,100 cells of a cylinder's band against 6 us): one block, cells t, t + 1024,
-// ... per thread, then a fixed-order block reduction.
+// are two, of which the second waits for the first): one block, cells t, t + 1024,
+// ... per thread, then a fixed-order block reduction.  One block's loads are
+// the limit: queued force records of 2,025 / 8,100 / 12,100 / 14,400 FP64 cells take
+// 6.3 / 8.3 / 9.6 / 10.3 us against 10.3 us in two launches, and ilbm_force_integrals
+// (which waits) 20 / 27 / 27 / 27 against 27 us (B200).
 constexpr int kSmallThreads = 1024;
-constexpr int64_t kSmallCells = 16 * kSmallThreads;
+constexpr int64_t kSmallCells = 12 * kSmallThreads;
 template <class R>
 __global__ void __launch_bounds__(kSmallThreads) k_force_small(RegionArgs a, const R *F, double *out,
                                                                const double *fsum, const int *status,
