@@ -1007,13 +1007,37 @@ static void launch_vectors(ilbm_ctx *ctx, const StepArgs &a_in, cudaStream_t st,
   }
 }
 
-// (singly: a body's band, where every cell reads force arrays: the cell form's
-// larger number of threads hides those scattered loads better, 23 against 28 us
-// for the 358k cells of the two-level sphere's band)
+// Launches that the cell form takes in rows that start on vectors too (B200, us
+// per level step, vector / cell form):
+//   - few cells, whose time is one thread's chain and not the traffic.  With a
+//     reflecting y or z face a warp of the vector form walks its cells one after
+//     another: up to 2^17 cells (D2Q9 98k 8.2 / 6.2 FP32, 9.1 / 6.2 FP16; D3Q19
+//     131k 12.4 / 9.3 and 18.5 / 12.4; D3Q27 131k 12.4 / 12.4 and 18.4 / 18.2, and at
+//     393k 24.1 / 24.3 and 32.2 / 39.1).  Without one, FP32 up to 2^15 cells (D2Q9 25k
+//     6.2 / 4.3, D3Q19 33k 8.3 / 6.2, D3Q27 9.3 / 6.2; with a flow's ghost shell D3Q19
+//     33k 10.3 / 10.1, 61k 9.3 / 10.3); the FP16 vectors' fewer accesses win from
+//     the start (D3Q27 15k 8.3 / 10.0)
+//   - D3Q19 FP32 with stored macro fields and force arrays on every cell, eleven
+//     scattered loads per cell (2.4 M cells 100 / 91)
+//   - a body's band (singly), where every cell reads force arrays: 23 against 28
+//     us for the 358k cells of the two-level sphere's band
+template <class L, int S>
+static bool prefers_cells(const StepArgs &a) {
+  int64_t cells = 1;
+  bool wall = false, all_forced = a.macro_in && !a.use_mbox && a.force;
+  for (int d = 0; d < L::D; ++d) {
+    cells *= a.rhi[d] - a.rlo[d] + 1;
+    if (d > 0) wall = wall || a.face_lo[d] == FACE_REFLECT || a.face_hi[d] == FACE_REFLECT;
+    all_forced = all_forced && a.flo[d] <= a.rlo[d] && a.fhi[d] >= a.rhi[d];
+  }
+  if (cells <= (wall ? 1 << 17 : (S == ILBM_STORAGE_F32_SHIFT ? 1 << 15 : 0))) return true;
+  return L::Q == 19 && S == ILBM_STORAGE_F32_SHIFT && all_forced;
+}
+
 template <class L, int S>
 void launch_cells(ilbm_ctx *ctx, const StepArgs &a, cudaStream_t st, bool with_ghosts, bool singly) {
   constexpr int V = StepVec<L, S>::value;
-  if (V > 1 && !singly && vec_width<L, S>(a) == V)
+  if (V > 1 && !singly && !prefers_cells<L, S>(a) && vec_width<L, S>(a) == V)
     launch_vectors<L, S, V>(ctx, a, st, with_ghosts);
   else
     launch_vectors<L, S, 1>(ctx, a, st, with_ghosts);
