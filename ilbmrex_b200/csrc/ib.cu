@@ -49,8 +49,23 @@ int level_step_split(ilbm_ctx *ctx, const ilbm_box &b, const ilbm_level_params *
 
 using namespace ilbm;
 
-// (ib_chain.cuh) bodies whose forcing chain is one launch
-static constexpr int kChainMaxMarkers = 512, kChainMaxCg = 448;
+// (ib_chain.cuh) bodies whose forcing chain is one launch.  Measured (B200, us per
+// step with its body, a launch per stage / the chain):
+//   2D: the chain's 256 warps take 512 markers in two rounds; 512 markers FP64 43.5 /
+//   31.8, FP32 34.6 / 28.3, FP16 36.6 / 30.8; a third round is a draw or a loss in
+//   the 2-byte form (576 markers 45.1 / 43.0, 36.6 / 33.8, 36.8 / 40.2) and the stored
+//   inverse soon is in every form (1,000 markers 49.8 / 56.0, 39.3 / 44.3, 39.1 / 48.1).
+//   3D: a marker forms rho and u at 125 cells, so one round is the limit (FP64
+//   D3Q19, 254 markers 70.8 / 66.3, 314 71.4 / 85.4), and the 4- and 2-byte forms,
+//   whose stages cost half as much, gain from it with the stored inverse in
+//   D3Q19 FP32 only (154 markers 40.0 / 31.4; explicit 40.6 / 44.1, D3Q27 39.7 / 43.5,
+//   FP16 41.0 / 44.7).
+//   An operator rebuilt every step gains in all of them as long as its rows fit the
+//   blocks' shared memory with room to spare (448 markers FP32 94 / 42, FP64 146 / 76;
+//   496 would fit in 3D).
+//   Bands up to 65,536 cells, which the chain clears: 61,009 cells FP32 37 / 28 (beyond,
+//   up to the 368,449 cells measured, it is still ahead: 45 / 38).
+static constexpr int kChainMaxMarkers = 512, kChainMaxMarkers3d = 256, kChainMaxCg = 448;
 static constexpr int64_t kChainMaxBand = 65536;
 static constexpr size_t kChainSharedMax = 224 * 1024;  // dynamic shared memory of a block
 
@@ -2642,6 +2657,15 @@ static int ib_box_table(ilbm_ib *ib, const ilbm_box *boxes, int nbox, const ilbm
 static int launch_chain(ilbm_ib *ib, const ilbm_box &box, const ilbm_level_params *lp, const IBArgs &a,
                         int mode, cudaStream_t s);
 
+// the most markers a body may have to take the chain (mode: 0 explicit, 1 stored
+// inverse, 2 operator rebuilt and solved by CG every step)
+static int chain_markers(const ilbm_ctx *ctx, int mode) {
+  if (mode == 2) return kChainMaxCg;
+  if (ctx->dim == 2) return kChainMaxMarkers;
+  if (ctx->storage == ILBM_STORAGE_F64) return kChainMaxMarkers3d;
+  return ctx->storage == ILBM_STORAGE_F32_SHIFT && ctx->q == 19 && mode == 1 ? kChainMaxMarkers3d : 0;
+}
+
 static int ib_update(ilbm_ib *ib, const ilbm_box *boxes, int nbox, const ilbm_level_params *lp,
                      double dt, double time, cudaStream_t s, bool defer_sum) {
   if (!ib || !boxes || nbox < 1 || !lp) {
@@ -2699,10 +2723,10 @@ static int ib_update(ilbm_ib *ib, const ilbm_box *boxes, int nbox, const ilbm_le
   // stages replace the band's ghost velocities by their periodic images
   // (FillBoundary, IBMarkerDF.cpp:702-703); the chain reads the ghosts as given.
   const bool images = periodic_band && box->macro_in && lp->ghost_mode != ILBM_GHOST_SELF;
-  if (ib->chain && !multi && single_ && !in_place && !images &&
-      ib->n <= (ivc_ && !use_dense_ ? kChainMaxCg : kChainMaxMarkers) &&
+  const int mode = !ivc_ ? 0 : (use_dense_ ? 1 : 2);
+  if (ib->chain && !multi && single_ && !in_place && !images && ib->n <= chain_markers(ctx, mode) &&
       (!ivc_ || (use_dense_ ? ib->dense_ready : (ib->moving || ib->p.ivc_rebuild_matrix > 0)))) {
-    int rc = launch_chain(ib, *box, lp, make_args(ib, dt, time), !ivc_ ? 0 : (use_dense_ ? 1 : 2), s);
+    int rc = launch_chain(ib, *box, lp, make_args(ib, dt, time), mode, s);
     if (rc) return rc;
     ib->csr_ready = ib->csr_ready || (ivc_ && !use_dense_);  // (a batch rebuilds such an operator itself)
     ib->fsum_deferred = false;

@@ -51,3 +51,28 @@ def test_small_bodies_take_the_cluster(n, chain):
     took = s.ctx.launches() - before
     assert (took == 3) if chain else (took >= 6)
     s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("q,storage,coupling,D,chain", [
+    (19, "f64", 0, 9.0, True), (19, "f64", 1, 10.0, False), (19, "f32", 1, 9.0, True), (19, "f32", 0, 9.0, False),
+    (19, "f32", 1, 10.0, False), (27, "f32", 1, 9.0, False), (19, "f16", 1, 9.0, False)])
+def test_spheres_that_take_the_cluster(q, storage, coupling, D, chain):
+    """3D: up to 256 markers (diameter 9: 254) in FP64, and in D3Q19 FP32 with the
+    stored inverse."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    from ilbmrex_b200 import cases
+    from ilbmrex_b200.lattice import D3Q19, D3Q27
+    from ilbmrex_b200.level import LevelSolver
+    case, ib, init = cases.sphere(36, 30, 28, D=D, center=(15.2, 14.9, 13.7), U=0.04, Re=30.0, coupling=coupling,
+                                  lattice=D3Q19 if q == 19 else D3Q27)
+    s = LevelSolver(case, storage, ib=ib)
+    s.set_macro(*init())
+    s.step(2)
+    before = s.ctx.launches()
+    s.step(1)
+    took = s.ctx.launches() - before
+    assert (took == 3) if chain else (took >= 6)
+    s.close()
