@@ -2567,12 +2567,15 @@ static double ivc_cg_tolerance(int storage) {
   return 1.0e-6;
 }
 
+// systems up to this size are solved by one block (launch_cg), larger ones by the grid
+constexpr int kOneBlockCg = 1024;
+
 // IVC solve by CG on the CSR operator (moving markers, rebuilt or large systems)
 static int launch_cg(ilbm_ib *ib, const IBArgs &a_in, cudaStream_t s) {
   ilbm_ctx *ctx = ib->ctx;
   IBArgs a = a_in;
   const double cg_tol = ivc_cg_tolerance(ctx->storage);
-  if (ib->n <= 1024) {
+  if (ib->n <= kOneBlockCg) {
     k_ivc_cg<<<1, kCgThreads, 0, s>>>(a, ib->d_xyz, ib->d_tgt, ib->d_uvw, ib->d_rowptr, ib->d_col,
                                       ib->d_val, ib->d_diag, ib->d_X, ib->d_Xh, ib->d_hist,
                                       ib->d_work, ib->d_F, 500, cg_tol, ib->d_status, ib->d_iters);
@@ -2805,11 +2808,12 @@ static int ib_update(ilbm_ib *ib, const ilbm_box *boxes, int nbox, const ilbm_le
       if (!ib->csr_ready || ib->moving || ib->p.ivc_rebuild_matrix > 0) {
         const int cb = std::min(4096, (ib->n * 32 + 255) / 256);
         k_csr_count<<<cb, 256, 0, s>>>(a, ib->d_xyz, ib->d_rowptr, tc);
-        cudaMemsetAsync(ib->d_rowmax, 0, sizeof(double), s);
+        // (the row sums serve the grid solve only)
+        double *rowmax = ib->n > kOneBlockCg ? ib->d_rowmax : nullptr;
+        if (rowmax) cudaMemsetAsync(rowmax, 0, sizeof(double), s);
         k_csr_scan<<<1, 1024, 0, s>>>(ib->n, ib->d_rowptr, ib->nnz_cap, ib->d_status);
         k_csr_fill<<<cb, 256, 0, s>>>(a, ib->d_xyz, ib->p.ivc_diag_reg, ib->d_rowptr, ib->d_col,
-                                      ib->d_val, ib->d_diag, ib->nnz_cap, ib->d_status, tw, tc,
-                                      ib->d_rowmax);
+                                      ib->d_val, ib->d_diag, ib->nnz_cap, ib->d_status, tw, tc, rowmax);
         ctx->launches += 3;
         ib->csr_ready = true;
       }
