@@ -610,6 +610,26 @@ static int vec_width_of(const ilbm_ctx *, const StepArgs &a, int *V) {
 
 uint32_t batch_per_block(int V, int w) { return step_vectors_per_block(V, (uint32_t)w); }
 
+// A batch of few cells in all takes the cell form, as a single small level does
+// (prefers_cells): up to 2^16, 2^17 where a case has a reflecting y or z face (B200,
+// us per step, vector / cell form: 4 Taylor-Green boxes of 64 x 64 FP32 8.3 / 7.2, 16 of
+// them 8.6 / 8.3, 24 9.3 / 8.5, 48 10.3 / 12.4; FP16 9.3 / 8.3, 9.3 / 9.3, 9.3 / 10.3, 10.7 /
+// 15.5; 4 channels of 256 x 128 11.4 / 9.3 FP32 and 15.5 / 12.4 FP16, 16 of them 16.5 /
+// 16.5 and 21.6 / 20.6, 24 18.5 / 22.6 and 23.9 / 29.8).  args: both buffer parities.
+static bool batch_prefers_cells(const ilbm_ctx *ctx, const StepArgs *args, int n) {
+  int64_t total = 0;
+  bool wall = false;
+  for (int c = 0; c < n / 2; ++c) {
+    int64_t cells = 1;
+    for (int d = 0; d < ctx->dim; ++d) {
+      cells *= args[c].rhi[d] - args[c].rlo[d] + 1;
+      if (d > 0) wall = wall || args[c].face_lo[d] == FACE_REFLECT || args[c].face_hi[d] == FACE_REFLECT;
+    }
+    total += cells;
+  }
+  return total <= (wall ? 1 << 17 : 1 << 16);
+}
+
 // the vector sequences of the cases' cells, V cells per vector for all of them
 int batch_plan(const ilbm_ctx *ctx, StepArgs *args, int n, int *V) {
   *V = 0;
@@ -618,6 +638,7 @@ int batch_plan(const ilbm_ctx *ctx, StepArgs *args, int n, int *V) {
     if (rc) return rc;
     *V = (*V == 0) ? v : std::min(*V, v);
   }
+  if (batch_prefers_cells(ctx, args, n)) *V = 1;
   for (int c = 0; c < n; ++c) {
     const StepArgs &a = args[c];
     int64_t vectors = (a.rhi[0] - a.rlo[0] + *V) / *V;  // (a self-filled box: its rows start on vectors)

@@ -82,3 +82,28 @@ def test_status_is_the_last_steps(tmp_path):
         B.progress()
     other.close()
     B.close()
+
+
+@pytest.mark.parametrize("storage", ["f32", "f16"])
+@pytest.mark.parametrize("wall,ncase", [(False, 1), (False, 16), (False, 17), (True, 4), (True, 5)])
+def test_small_batches_keep_the_single_levels_bits(storage, wall, ncase):
+    """Batches on both sides of the cell form's limits (2^16 cells, 2^17 with
+    reflecting walls): bit for bit the levels alone."""
+    def make():
+        return cases.channel_bounce_back(nx=256, ny=128) if wall else cases.taylor_green(64, U0=0.02, tau=0.7)
+
+    B = Batch(D2Q9, storage)
+    ids = []
+    for _ in range(ncase):
+        case, init = make()
+        ids.append(B.add(B.solver(case, None, init), max_steps=8))
+    B.step(4)
+    case, init = make()
+    ref = LevelSolver(case, storage)
+    ref.set_macro(*init())
+    ref.step(5)
+    want = ref.get_f()
+    for cid in ids:
+        np.testing.assert_array_equal(B.sync(cid).get_f(), want)
+    ref.close()
+    B.close()
