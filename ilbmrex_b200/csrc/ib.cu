@@ -1909,8 +1909,7 @@ __global__ void k_fill_boundary(IBArgs a, double *EV) {
 template <class R>
 __device__ __forceinline__ void export_cell(const IBArgs &a, const double *EFT, const double *RHO,
                                             R *F, int mgl0, int mgl1, int mgl2, int64_t ms0,
-                                            int64_t ms1, int64_t ms2, int64_t t,
-                                            double *stored = nullptr) {
+                                            int64_t ms1, int64_t ms2, int64_t t) {
   const int i = a.blo[0] + (int)(t % a.bn[0]);
   const int j = a.blo[1] + (int)((t / a.bn[0]) % a.bn[1]);
   const int k = a.blo[2] + (int)(t / ((int64_t)a.bn[0] * a.bn[1]));
@@ -1920,19 +1919,9 @@ __device__ __forceinline__ void export_cell(const IBArgs &a, const double *EFT, 
   if (!inside) return;
   const int64_t m = (int64_t)(i - mgl0) + (int64_t)(j - mgl1) * ms0 + (int64_t)(k - mgl2) * ms1;
   const double dr = X::mul(a.dt, RHO[t]);
-  const R fx = R(X::mul(dr, EFT[t])), fy = R(X::mul(dr, EFT[t + a.nb]));
-  F[m] = fx;
-  F[m + ms2] = fy;
-  R fz = R(0);
-  if (a.dim == 3) {
-    fz = R(X::mul(dr, EFT[t + 2 * a.nb]));
-    F[m + 2 * ms2] = fz;
-  }
-  if (stored) {  // the values as stored (the force region is the band inside the domain)
-    stored[0] = double(fx);
-    stored[1] = double(fy);
-    stored[2] = double(fz);
-  }
+  F[m] = R(X::mul(dr, EFT[t]));
+  F[m + ms2] = R(X::mul(dr, EFT[t + a.nb]));
+  if (a.dim == 3) F[m + 2 * ms2] = R(X::mul(dr, EFT[t + 2 * a.nb]));
 }
 
 template <class R>
@@ -3162,7 +3151,7 @@ struct IBCase {
   IBArgs a;
   double *xyz;
   const double *ref;
-  double *tgt, *uvw, *F, *EV, *EFI, *RHO, *fsum;
+  double *tgt, *uvw, *F, *EFI, *fsum;
   int *status, *iters;
   int mode;     // 0 explicit, 1 stored inverse, 2 CG
   int rebuild;  // CG operator rebuilt every step (moving markers / ivc_rebuild_matrix)
@@ -3474,7 +3463,7 @@ struct IBBatch {
   int nc = 0, rec_slots = 1;
   std::vector<void *> allocs;
   IBCase *d_cases = nullptr;
-  int64_t total_m = 0, total_b = 0, total_drows = 0, total_rm = 0;
+  int64_t total_m = 0, total_drows = 0, total_rm = 0;
   int nbt = 0;  // band tiles
   // work lists: every marker, the markers of bodies whose operator is
   // rebuilt each step, every row of a stored inverse (case, item), and the
@@ -3486,7 +3475,7 @@ struct IBBatch {
   int *d_clcase = nullptr;
   int ncl = 0;
   size_t cl_shared = 0;
-  bool any_periodic = false, any_explicit = false, any_rebuild = false;
+  bool any_periodic = false, any_explicit = false;
   int *d_steps = nullptr, *d_limit = nullptr;
   double *d_rec = nullptr, *d_tpart = nullptr;  // record rings; the export's tile partials
   // fork / join of the moving bodies' operator build and CG (on the context's
@@ -3577,7 +3566,7 @@ int ib_batch_create(ilbm_ctx *ctx, const std::vector<IBBatchCase> &cases, int re
   b->nc = (int)cases.size();
   b->rec_slots = std::max(1, rec_slots);
   std::vector<IBCase> hc(b->nc);
-  std::vector<int64_t> moff(b->nc + 1, 0), boff(b->nc + 1, 0);
+  std::vector<int64_t> moff(b->nc + 1, 0);
   std::vector<int> cgcase, clcase;
   std::vector<ItemRef> mlist, rlist, dlist, btiles;
   std::vector<std::vector<double>> kin(b->nc);
@@ -3586,7 +3575,6 @@ int ib_batch_create(ilbm_ctx *ctx, const std::vector<IBBatchCase> &cases, int re
     std::memset(&k, 0, sizeof(k));
     ilbm_ib *ib = cases[c].ib;
     moff[c + 1] = moff[c];
-    boff[c + 1] = boff[c];
     b->status_ptrs.push_back(nullptr);
     if (!ib) continue;
     if (ib->ctx != ctx) {
@@ -3611,9 +3599,7 @@ int ib_batch_create(ilbm_ctx *ctx, const std::vector<IBBatchCase> &cases, int re
     k.tgt = ib->d_tgt;
     k.uvw = ib->d_uvw;
     k.F = ib->d_F;
-    k.EV = ib->d_EV;
     k.EFI = ib->d_EFI;
-    k.RHO = ib->d_RHO;
     k.fsum = ib->d_fsum;
     k.status = ib->d_status;
     k.iters = ib->d_iters;
@@ -3656,7 +3642,6 @@ int ib_batch_create(ilbm_ctx *ctx, const std::vector<IBBatchCase> &cases, int re
       k.kin_steps = ns;
     }
     moff[c + 1] = moff[c] + ib->n;
-    boff[c + 1] = boff[c] + ib->nb;
     const bool cluster = clusters && k.mode == 2;
     for (int m = 0; m < ib->n; ++m) {
       mlist.push_back({c, m});
@@ -3675,7 +3660,6 @@ int ib_batch_create(ilbm_ctx *ctx, const std::vector<IBBatchCase> &cases, int re
     cudaMemsetAsync(ib->d_EFI, 0, 3 * (size_t)ib->nb * sizeof(double), ctx->stream);
     b->any_periodic = b->any_periodic || k.periodic_band;
     b->any_explicit = b->any_explicit || k.mode == 0;
-    b->any_rebuild = b->any_rebuild || k.rebuild;
     b->status_ptrs.back() = ib->d_status;
   }
   int rc;
@@ -3704,7 +3688,6 @@ int ib_batch_create(ilbm_ctx *ctx, const std::vector<IBBatchCase> &cases, int re
   b->d_rec = rec;
   for (int c = 0; c < b->nc; ++c) hc[c].rec = rec + (size_t)c * b->rec_slots * 8;
   b->total_m = moff.back();
-  b->total_b = boff.back();
   {
     double *tw = nullptr;
     int4 *tc = nullptr;

@@ -410,8 +410,7 @@ bool plan_vectors(StepArgs &a, int dim, int V) {
 }
 
 template <class L, int S>
-static int launch_step(ilbm_ctx *ctx, const StepArgs &a, const ilbm_level_params *p) {
-  (void)p;
+static int launch_step(ilbm_ctx *ctx, const StepArgs &a) {
   launch_cells<L, S>(ctx, a, ctx->stream, true);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "level step launch");
@@ -968,7 +967,7 @@ int level_step_impl(ilbm_ctx *ctx, const ilbm_box *boxes, int nbox, const ilbm_l
       }
     }
     if (part == 0) {
-      rc = ILBM_DISPATCH(ctx, launch_step, ctx, a, p);
+      rc = ILBM_DISPATCH(ctx, launch_step, ctx, a);
     } else if (a.hi[ctx->dim - 1] == a.lo[ctx->dim - 1]) {
       // one cell along the split dimension: the first part takes it all
       if (part == 1) rc = ILBM_DISPATCH(ctx, launch_step_part, ctx, a, true);
