@@ -3547,22 +3547,31 @@ int ib_batch_create(ilbm_ctx *ctx, const std::vector<IBBatchCase> &cases, int re
   // (its operator rebuilt each step, its rows within the blocks' shared memory)
   // and they run in two waves at most; else the sparse operators and a block
   // each, in one set of launches for all.  Both kinds in a row, or a third wave,
-  // cost more than the clusters give.  Measured (B200, 15 clusters a wave, us per
-  // step with clusters / without): 15 bodies of 240 markers 56 / 77 FP32, 96 / 130
-  // FP64; 28 of them 102 / 111 and 178 / 172; 32 of 200 markers 125 / 111 and 223 / 172;
+  // cost more than the clusters give, except in the 4- and 2-byte forms (fewer
+  // iterations) where the bodies are large or as many stored inverses, whose rows
+  // fill the device, are applied beside them: then three waves.  Measured (B200, 15 clusters a wave, us per step with clusters /
+  // without): 15 bodies of 240 markers 56 / 77 FP32, 96 / 130 FP64; 28 of them 98 / 107
+  // and 177 / 170; 32 of them 129 / 123 and 222 / 181, with 32 fixed bodies 161 / 167 and
+  // 279 / 248; 48 with 48 219 / 216; 40 of 240 markers 141 / 137, of 384 167 / 179 FP32;
   // 12 bodies of 200 and 420 markers by turns 106 / 91 and 196 / 158.
   bool clusters = true;
-  int nclusters = 0;
+  int nclusters = 0, ndense = 0;
+  int64_t markers = 0;
   for (const IBBatchCase &x : cases) {
     const ilbm_ib *ib = x.ib;
-    if (!ib || batch_mode(ib) != 2) continue;
+    if (!ib) continue;
+    ndense += batch_mode(ib) == 1;
+    if (batch_mode(ib) != 2) continue;
     const size_t sh = chain_shared(2, ib->n, ib->dim, kBatchCgCtas);
     clusters = clusters && batch_rebuilds(ib) && sh <= kChainSharedMax;
     b->cl_shared = std::max(b->cl_shared, sh);
+    markers += ib->n;
     ++nclusters;
   }
+  const bool third = ndense >= nclusters || markers >= 300 * (int64_t)nclusters;
+  const int waves = ctx->storage != ILBM_STORAGE_F64 && third ? 3 : 2;
   clusters = clusters && nclusters > 0 &&
-             nclusters <= 2 * clusters_of(k_b_cluster_cg, kBatchCgCtas, b->cl_shared, kChainSharedMax);
+             nclusters <= waves * clusters_of(k_b_cluster_cg, kBatchCgCtas, b->cl_shared, kChainSharedMax);
   b->nc = (int)cases.size();
   b->rec_slots = std::max(1, rec_slots);
   std::vector<IBCase> hc(b->nc);
