@@ -146,8 +146,9 @@ __global__ void k_final_sum(const double *partial, int nparts, double *out,
 // are two, of which the second waits for the first): one block, cells t, t + 1024,
 // ... per thread, then a fixed-order block reduction.  One block's loads are
 // the limit: queued force records of 2,025 / 8,100 / 12,100 / 14,400 FP64 cells take
-// 6.3 / 8.3 / 9.6 / 10.3 us against 10.3 us in two launches, and ilbm_force_integrals
-// (which waits) 20 / 27 / 27 / 27 against 27 us (B200).
+// 6.3 / 8.3 / 8.5 / 10.3 us against 10.3 us in two launches, and ilbm_force_integrals
+// (which waits) 20 / 25 / 28 / 28 against 24 us (B200): past 7,000 cells the records, taken
+// every step, are what the limit goes by, for both sum in one order.
 constexpr int kSmallThreads = 1024;
 constexpr int64_t kSmallCells = 12 * kSmallThreads;
 template <class R>

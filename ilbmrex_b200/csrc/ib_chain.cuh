@@ -6,11 +6,12 @@
 // own (up to ten kernels and three memsets of 2-5 us, each waiting for the one
 // before) they are bound by launch latency on the device and by API calls on
 // the host.  Here one cluster of kChainCtas blocks runs them with a cluster
-// barrier between stages.  Measured (B200, per step): the 1024 x 512 FP32
-// cylinder (126 markers) 56 -> 41 us with its record, host time 49 -> 27 us; the
-// pitching airfoil (240 markers, operator rebuilt) 117 -> 72 us; the finest
-// level of the three-level cylinder (504 markers) 4 x 26 us of stages -> 4 x
-// 20 us.  Eight blocks measured 51 us instead of 32 us cold on the last.
+// barrier between stages.  Measured (B200, per step, with the stages' later
+// changes): the 1024 x 512 FP32 cylinder (126 markers) 56 -> 36 us with its
+// one-launch record; the pitching airfoil (240 markers, operator rebuilt) 115 ->
+// 64 us; the finest level of the three-level cylinder (503 markers) 4 x 26 us of
+// stages -> 4 x 21 us.  Eight blocks measured 51 us instead of 33 us cold on the
+// last.  Which bodies take it: chain_markers (ib.cu).
 //
 // Stages:
 //   1  a warp per marker: its position (moving bodies), kernel weights, the

@@ -246,7 +246,8 @@ __device__ __forceinline__ void moments64(const double *f, double Fx, double Fy,
 // are redone with the functions above.  About 350 FP64 instructions per D3Q19
 // cell instead of about 650, which FP64 steps are bound by beside the memory
 // traffic: the D3Q19 step of the 128 x 64 x 64 sphere 50 -> 37 us (24.7 us of
-// traffic), its body's band with forces 25 -> 7 us.
+// traffic; 39 us as one launch without its body, 78 us before with the ghost
+// shell's old push), its body's band with forces 25 -> 7 us.
 // ---------------------------------------------------------------------------
 struct Tau64 {
   double tau, inv;  // tau and 1 / tau rounded to nearest

@@ -21,7 +21,7 @@ namespace ilbm {
 // shell is one sequence of cells: slab d holds the cells outside the box in
 // dimension d, inside it in the active dimensions below d, and on the grown
 // range of the others (StepArgs::goff, filled by ghost_offsets).
-// The work runs in the leading blocks of the k_step launch (it writes only
+// The work runs in blocks spread among those of the k_step launch (it writes only
 // slots that no cell's push writes, and reads only f^n), so its strided
 // accesses overlap the main stream instead of preceding it.  It is bound by
 // latency: one thread's chain is one ghost's index, its loads in flight
@@ -241,15 +241,16 @@ __device__ __noinline__ void ghost_push(const StepArgs &a, const int (*lb)[6], u
 // instructions per D3Q19 FP32 cell on rows whose x faces are periodic; four
 // cells per thread (128 registers, 16 warps) hold 155 KB and issue 330, the
 // arithmetic halved by the packed instructions and the address and index work
-// shared by four cells.  Measured (B200, per level step): the 512 x 128 x 128
-// FP32 duct 314 -> 213 us (0.63 -> 0.93 of the copy bandwidth), the 256 x 128 x
-// 128 FP16 sphere 154 -> 102 us alone, the D3Q27 FP32 sphere 150 x 75 x 83
-// 61 -> 45 us, 2.1 M cells of the D3Q19 FP32 sphere 68 -> 57 us.
+// shared by four cells.  Measured (B200): the 512 x 128 x 128 FP32 duct 313 ->
+// 217 us per step (0.63 -> 0.92 of the copy bandwidth); the step alone, repeated, of
+// the 256 x 128 x 128 level of the D3Q19 sphere 124 -> 104 us FP32 and 148 -> 94 us
+// FP16, of the D3Q27 FP32 sphere 150 x 75 x 83 64 -> 48 us, of 2.1 M D3Q19 FP32
+// cells 65 -> 57 us.
 template <class L, int S>
 struct StepVec {
   // 16 bytes per FP32 access; two cells for D3Q27, whose 27 populations of four
   // cells do not fit the registers; eight cells of FP16 spill (119 us against
-  // 102 us for four).  FP64 is bound by its arithmetic as well and stays with
+  // 102 us for four in one build).  FP64 is bound by its arithmetic as well and stays with
   // one cell: two cells per thread spilled (437 against 389 us for two steps
   // of the 128 x 64 x 64 sphere).
   static constexpr int value = S == ILBM_STORAGE_F64 ? 1 : (L::Q <= 19 ? 4 : 2);

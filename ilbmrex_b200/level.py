@@ -281,7 +281,9 @@ class LevelSolver:
         """_box for the step loop: the struct made last time for the same
         addresses and strides (a step alternates between two), which callers
         do not change.  Filling one anew takes longer than a small level's step
-        on the device (channel 64 x 48: 11.4 -> 9.5 us, Taylor-Green 256 x 256: 8.5 -> 6.5 us per step with it held)."""
+        on the device (channel 64 x 48: 10.7 -> 9.7 us, Taylor-Green 256 x 256:
+        8.2 -> 6.7 us per step with it held); a solver's first two steps, which
+        fill both, pay the key (about 1 us) on top."""
         ptr = lambda t: t.data_ptr() if t is not None else 0
         key = (ptr(f_in), ptr(f_out), ptr(macro_in), ptr(macro_out), ptr(force), ptr(force_prev),
                self.f.stride(), self.macro.stride())
