@@ -372,7 +372,8 @@ int launch_cf_fill(ilbm_ctx *ctx, const CFArgs &g) {
 template <class L, int S>
 int launch_avg_down(ilbm_ctx *ctx, const AvgArgs &g) {
   int64_t n = 1;
-  for (int d = 0; d < L::D; ++d) n *= (int64_t)(g.chi_box[d] - g.clo_box[d] + 1);
+  for (int d = 0; d < L::D; ++d) n *= std::max<int64_t>(0, (int64_t)(g.chi_box[d] - g.clo_box[d] + 1));
+  if (n == 0) return ILBM_OK;  // a box of no cells
   if (n > INT32_MAX) {
     set_error("fine box too large: it covers 2^31 coarse cells or more");
     return ILBM_ERR_RANGE;

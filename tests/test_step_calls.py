@@ -102,3 +102,37 @@ def test_batched_case_of_very_many_cells(nx, ny):
         assert torch.equal(one[q, 0, 1:-1, 1:-1], two[q, 0, 1:-1, 1:-1])
     ctx.L.ilbm_batch_destroy(h)
     ctx.close()
+
+
+def test_average_down_of_an_empty_box():
+    """A fine box of no cells on a level in between: nothing to average, and the
+    next call on the context works."""
+    ctx = Context(D2Q9, "f64")
+    dev = torch.device("cuda")
+    f, m = torch.zeros((9, 1, 34, 34), device=dev, dtype=torch.float64), torch.zeros((4, 1, 36, 36), device=dev, dtype=torch.float64)
+    case = cases.LevelCase(D2Q9, (64, 64, 1), nu=0.06)
+
+    def box(lo, hi):
+        b = capi.Box_t()
+        for d in range(2):
+            b.lo[d], b.hi[d] = lo, hi
+        b.ngrow_f, b.ngrow_m = 1, 2
+        b.fstride[:] = [34, 34 * 34, 34 * 34]
+        b.mstride[:] = [36, 36 * 36, 36 * 36]
+        b.f_in, b.macro_in = f.data_ptr(), m.data_ptr()
+        return b
+
+    pc, pf = level_params(case, uniform_force=False), level_params(case, uniform_force=False)
+    pc.ghost_mode = pf.ghost_mode = capi.GHOST_CALLER
+    for d in range(2):
+        pf.domain_hi[d] = 2 * pc.domain_hi[d] + 1
+    coarse, fine = box(0, 31), box(16, 15)
+    torch.cuda.synchronize()
+    capi.check(ctx.L.ilbm_average_down(ctx.h, C.byref(coarse), C.byref(pc), C.byref(fine), C.byref(pf)), "average_down")
+    out = torch.zeros_like(f)
+    b = box(0, 31)
+    b.f_out, b.macro_in = out.data_ptr(), None
+    p = level_params(cases.LevelCase(D2Q9, (32, 32, 1), nu=0.06), uniform_force=False)
+    capi.check(ctx.L.ilbm_level_step(ctx.h, C.byref(b), 1, C.byref(p)), "level_step")
+    ctx.sync()
+    ctx.close()
