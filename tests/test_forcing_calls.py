@@ -71,3 +71,22 @@ def test_caller_filled_band_over_a_periodic_face(n):
     np.testing.assert_array_equal(out[0], out[1])
     np.testing.assert_array_equal(f.cpu().numpy(), out[1])
     s.close()
+
+
+@pytest.mark.parametrize("center", [(15.2, 2.4, 13.7), (15.2, 14.9, 26.1), (15.2, 1.2, 0.8)])
+def test_sphere_over_a_periodic_face(center):
+    """The 3D chain's band beyond periodic faces, an edge of two among them:
+    explicit coupling against the oracle."""
+    from oracle.checker import CpuLevel
+    case, ib, init = cases.sphere(36, 30, 28, D=8.0, center=center, U=0.04, Re=30.0, coupling=0)
+    cpu = CpuLevel(case, "oracle")
+    cpu.set_macro(*init())
+    cpu.init_equilibrium()
+    cpu.ib_create(ib)
+    cpu.step(4)
+    s = LevelSolver(case, "f64", ib=ib)
+    s.set_macro(*init())
+    s.step(4)
+    f, g = s.get_f(), cpu.get_f()
+    assert np.sqrt(np.sum((f - g) ** 2) / np.sum(g ** 2)) <= 1e-12
+    s.close()
