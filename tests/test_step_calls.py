@@ -68,6 +68,8 @@ def test_box_of_very_many_cells(nx, ny):
         assert torch.equal(outs[0][q, 0, 1:-1, 1:-1], outs[1][q, 0, 1:-1, 1:-1])
     assert float(outs[0][1, 0, -2, 1:-1].abs().max()) > 0.0
     ctx.close()
+    del fi, fo, outs
+    torch.cuda.empty_cache()
 
 
 @pytest.mark.parametrize("nx,ny", [(1024, 96), (32771, 32800)])
@@ -102,6 +104,8 @@ def test_batched_case_of_very_many_cells(nx, ny):
         assert torch.equal(one[q, 0, 1:-1, 1:-1], two[q, 0, 1:-1, 1:-1])
     ctx.L.ilbm_batch_destroy(h)
     ctx.close()
+    del fi, one, two
+    torch.cuda.empty_cache()
 
 
 def test_average_down_of_an_empty_box():
