@@ -3372,6 +3372,7 @@ static void chain_case(ilbm_ib *ib, const IBArgs &a, int mode, IBCase &k) {
   k.X = ib->d_X;
   k.Xh = ib->d_Xh;
   k.hist = ib->d_hist;
+  k.nnz_cap = ib->nnz_cap;
   k.reg = ib->p.ivc_diag_reg;
   k.cg_tol = ivc_cg_tolerance(ib->ctx->storage);
   k.Ainv = ib->d_Ainv;

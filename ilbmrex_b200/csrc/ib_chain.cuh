@@ -182,6 +182,10 @@ __device__ __forceinline__ void chain_cg(cgrp::cluster_group &cl, const IBCase &
   double *x = p + 3 * n, *r = x + 3 * rows, *ap = r + 3 * rows, *b = ap + 3 * rows, *dg = b + 3 * rows;
   double *slot = dg + rows;  // [2][CTAS][6]
   double *tot = slot + 2 * CTAS * 6;
+  // the operator's entries over all blocks (rank 0's counts): beyond the capacity
+  // that the sparse operator has, the body is refused as it is there
+  __shared__ int entries;
+  if (tid == 0) entries = 0;
   cl.barrier_arrive();  // (waited for before the first remote write)
   // the step's weight table, and the start: zero, the last solution, or the
   // extrapolation of the last two
@@ -206,6 +210,7 @@ __device__ __forceinline__ void chain_cg(cgrp::cluster_group &cl, const IBCase &
   // the operator's rows
   const int rw = (nl + NW - 1) / NW, i0 = wid * rw, ni = max(0, min(nl - i0, rw));  // rw <= RW
   uint32_t chunks = 0;
+  int coupled = 0;
   for (int j0 = 0; j0 < n; j0 += 32) {
     const int j = j0 + lane;
     bool any = false;
@@ -215,12 +220,16 @@ __device__ __forceinline__ void chain_cg(cgrp::cluster_group &cl, const IBCase &
     if (j < n)
       for (int i = 0; i < ni; ++i) {
         const int row = r0 + i0 + i;
-        const double v = may_couple_tab(a, tc, row, j) ? ivc_entry_tab(a, tw, tc, row, j, k.reg, ws) : 0.0;
+        const bool c = may_couple_tab(a, tc, row, j);
+        const double v = c ? ivc_entry_tab(a, tw, tc, row, j, k.reg, ws) : 0.0;
+        coupled += c;
         A[(size_t)(i0 + i) * n + j] = v;
         if (row == j) dg[i0 + i] = v;
       }
   }
   cl.barrier_wait();  // every block of the cluster runs
+  for (int o = 16; o > 0; o >>= 1) coupled += __shfl_xor_sync(0xffffffffu, coupled, o);
+  if (lane == 0 && coupled) atomicAdd(cl.map_shared_rank(&entries, 0), coupled);  // (read after the next barrier)
   __syncthreads();
   // ap = A p on the block's rows
   auto product = [&]() {
@@ -331,6 +340,7 @@ __device__ __forceinline__ void chain_cg(cgrp::cluster_group &cl, const IBCase &
   if (rank == 0 && tid == 0) {
     *k.iters = it;
     if (!done) atomicOr(k.status, 4);
+    if (entries > k.nnz_cap) atomicOr(k.status, 2);
     *k.hist = (h + 1 < 2) ? h + 1 : 2;
   }
   if (own) {

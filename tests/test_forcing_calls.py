@@ -90,3 +90,35 @@ def test_sphere_over_a_periodic_face(center):
     f, g = s.get_f(), cpu.get_f()
     assert np.sqrt(np.sum((f - g) ** 2) / np.sum(g ** 2)) <= 1e-12
     s.close()
+
+
+@pytest.mark.parametrize("n,refused", [(240, False), (400, True), (440, True), (600, True)])
+def test_markers_too_dense_are_refused(n, refused):
+    """A rebuilt 2D operator holds 96 neighbours per row on average; on 31 cells of
+    circumference 240 markers have about 70, 400 about 120.  Alone and in a batch,
+    whichever solve takes them."""
+    from ilbmrex_b200.batch import Batch
+    from ilbmrex_b200.lattice import D2Q9
+    case, ib, init = cases.cylinder(nx=64, ny=48, D=10, center=(24.3, 23.6), U=0.05, Re=40, n_marker=n)
+    ib.ivc_rebuild_matrix = 1
+    B = Batch(D2Q9, "f32")
+    s, joined = B.solver(case, ib, init), False
+    try:
+        s.step(1)
+        for _ in range(2):
+            if refused:
+                with pytest.raises(capi.IlbmError, match="capacity"):
+                    s.step(1, record_force=True)
+            else:
+                s.step(1, record_force=True)
+        joined = B.add(s, max_steps=8) > 0
+        B.step(2)
+        if refused:
+            with pytest.raises(capi.IlbmError, match="capacity"):
+                B.progress()
+        else:
+            B.progress()
+    finally:
+        if not joined:
+            s.close()
+        B.close()
